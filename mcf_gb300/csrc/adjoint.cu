@@ -475,8 +475,8 @@ __global__ void __launch_bounds__(kAdjTPB)
     const double xj[3] = {xj4.x, xj4.y, xj4.z};
     double r[3];
     const double dd2 = exact_sep<D>(k, xi, xj, s_shift[sl * kAdjTPB + tid], r);
-    const double u = rsqrt(dd2);
-    const double dist = dd2 * u;
+    double u;
+    const double dist = root64<true>(dd2, u);
     double ev[3];
 #pragma unroll
     for (int a = 0; a < D; ++a) ev[a] = r[a] * u;
@@ -500,8 +500,8 @@ __global__ void __launch_bounds__(kAdjTPB)
       float z[6];
       pair_draw<D>(3, k.rk, step, pidi, tp.pid[j], z);
 #pragma unroll
-      for (int a = 0; a < D; ++a) gz[a] = (double)z[a];
-      sg = (double)z[5];
+      for (int a = 0; a < D; ++a) gz[a] = widen(z[a]);
+      sg = (z[5] < 0.0f) ? -1.0 : 1.0;
       const double arg = -4.0 * kt * f_d;
       const double rs = rsqrt(arg);
       f_r = arg * rs * inv_sqdt;
@@ -687,8 +687,9 @@ __global__ void __launch_bounds__(kAdjTPB)
     const double xj[3] = {xj4.x, xj4.y, xj4.z};
     double r[3];
     const double dd2 = exact_sep<D>(k, xi, xj, s_shift[sl * kAdjTPB + tid], r);
-    const double dist = sqrt(dd2);
-    const double f = (nbi + nbar[j]) * kernel_gradw<double>(k, dist) / dist;
+    double u;
+    const double dist = root64<true>(dd2, u);
+    const double f = (nbi + nbar[j]) * kernel_gradw<double>(k, dist) * u;
 #pragma unroll
     for (int a = 0; a < D; ++a) acc[a] += f * r[a];
   }

@@ -120,12 +120,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
           const double xj[3] = {xj4.x, xj4.y, xj4.z};
           double r[3];
           const double d2 = exact_sep<D>(k, xi, xj, t.shift[sl], r);
-          if (d2 >= k.rc2) continue;
+          if (beyond(d2, k.rc2)) continue;
           if (hs < 0 && (sl > CENTER || (sl == CENTER && q > li))) hs = kept;
           nl[(size_t)kept * n + i] = (uint16_t)ent;
           ++kept;
           if (acc_i) {
-            const double w = kernel_w<double>(k, sqrt(d2));
+            const double w = kernel_w<double>(k, root64(d2));
             sum += (k.rhs_density_type == 1) ? w * m[j] : w;
           }
         }
@@ -319,12 +319,12 @@ __global__ void __launch_bounds__(kReuseTPB)
       const double xj[3] = {xj4.x, xj4.y, xj4.z};
       double r[3];
       const double d2 = exact_sep<D>(k, xi, xj, s_shift[sl * kReuseTPB + tid], r);
-      if (d2 >= k.rc2) continue;
+      if (beyond(d2, k.rc2)) continue;
       if (hs < 0 && (sl > CENTER || (sl == CENTER && q > li))) hs = kept;
       if (kept < cap) nl[(size_t)kept * n + i] = (uint16_t)ent;
       ++kept;
       if (acc_i) {
-        const double w = kernel_w<double>(k, sqrt(d2));
+        const double w = kernel_w<double>(k, root64(d2));
         sum += (k.rhs_density_type == 1) ? w * m[j] : w;
       }
     }
@@ -437,8 +437,8 @@ __global__ void __launch_bounds__(kReuseTPB)
     // the kernel's argument is MCF's SQRT(DOT_PRODUCT(rij, rij)), correctly
     // rounded: near the cut-off W'(d) ~ (3 - d/h)^4 amplifies any rounding
     // difference of d by 4 d / (3h - d); 1/d only scales well-conditioned terms
-    const T inv_d = rsqrt(d2);
-    const T d = sqrt(d2);
+    T inv_d;
+    const T d = root64<true>(d2, inv_d);
     const double4_32a v4 = v[j];
     T vi[3] = {v4i.x, v4i.y, v4i.z};
     T vj[3] = {v4.x, v4.y, v4.z};
@@ -1054,8 +1054,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
             for (int a = 0; a < 3; ++a) rr[a] = (T)r64[a];
             // MCF's correctly rounded SQRT for the kernel's argument (see
             // k_force64)
-            inv_d = (T)rsqrt(d2);
-            d = (T)sqrt(d2);
+            double inv64;
+            d = (T)root64<true>(d2, inv64);
+            inv_d = (T)inv64;
             const double4_32a vj4 = v[j], cj4 = pc[j];
             vj[0] = (T)vj4.x; vj[1] = (T)vj4.y; vj[2] = (T)vj4.z;
             Aj = (T)cj4.x; Bj = (T)cj4.y; Cj = (T)cj4.z; Pj = (T)cj4.w;

@@ -1,6 +1,8 @@
 // sph.cuh -- SPH kernel, equation of state and pair force forms, templated
 // on the arithmetic type (double: FP64 path, float: FP32-mixed path).
 #pragma once
+#include <type_traits>
+
 #include "mcfg_internal.cuh"
 
 namespace mcfg {
@@ -22,8 +24,14 @@ struct KC<double> {
   // the kernel's argument s = r / h as MCF divides it
   // (kernel_kernel_quintic_spline.F90:69,177): near the cut-off W and W'
   // amplify a rounding difference of s by 4-5 s / (3 - s), so the FP64 path
-  // keeps MCF's division
-  __device__ static double arg(const Consts& k, double r) { return r / k.h; }
+  // keeps MCF's correctly rounded quotient.  h is a constant, so the
+  // division is Markstein's correction of r * (1/h) by its exact residual
+  // (IBM J. Res. Dev. 34, 1990; correctly rounded for a correctly rounded
+  // 1/h): 3 FP64 slots where the general division took about 10.
+  __device__ static double arg(const Consts& k, double r) {
+    const double q = r * k.inv_h;
+    return fma(fma(-q, k.h, r), k.inv_h, q);
+  }
   __device__ static double inv_h(const Consts& k) { return k.inv_h; }
   __device__ static double coef(const Consts& k) { return k.coef; }
   __device__ static double coef_grad(const Consts& k) { return k.coef_grad; }
@@ -42,12 +50,130 @@ struct KC<float> {
   __device__ static float eta_coef(const Consts& k) { return k.eta_coeff; }
 };
 
+// ---------------------------------------------------------------------------
+// FP64 arithmetic for GB300's narrow FP64 pipe (2 DFMA a clock per SM, 1/64 of
+// the FP32 rate): the FP64 sweeps are bound by the number of FP64 instructions
+// a pair issues, while the integer pipe idles.  So comparisons, selections
+// and widenings run on the bits, and square root, reciprocal root and the
+// kernel polynomials take the fewest FP64 operations that keep their rounding.
+// Measured on 64^3 particles: the FP64 step 9.18 -> 7.22 ms, the same error
+// against 64-bit references as the general sqrt, rsqrt, division and powers.
+// ---------------------------------------------------------------------------
+
+// d2 >= rc2 on the bits (both non-negative; a NaN separation is kept, as the
+// FP64 comparison keeps it)
+__device__ __forceinline__ bool beyond(double d2, double rc2) {
+  const long long b = __double_as_longlong(d2);
+  return b >= __double_as_longlong(rc2) && b <= 0x7ff0000000000000ll;
+}
+
+// FP32 -> FP64 on the integer pipe (exact; normal numbers and zero, which is
+// what Box-Muller with flush-to-zero gives)
+__device__ __forceinline__ double widen(float z) {
+  const unsigned u = __float_as_uint(z);
+  const unsigned mag = u & 0x7fffffffu;
+  const unsigned hi = mag ? (u & 0x80000000u) | ((mag >> 3) + 0x38000000u) : 0u;
+  return __hiloint2double((int)hi, (int)(u << 29));
+}
+
+// sqrt(a) and, with INV, 1/sqrt(a) from one seed: Goldschmidt's coupled
+// iteration on g -> sqrt(a), hh -> 1/(2 sqrt(a)) from the hardware's
+// approximation, then the residual a - g^2 (exact by FMA) corrects g, which
+// rounds to the nearest double but for cases within ~2^-26 ulp of a tie
+// (Markstein 1990; Cornea, Harrison, Tang 2002).  6 FP64 slots (8 with INV)
+// against about 17 of separate sqrt and rsqrt calls.  Zero, tiny, infinite and
+// NaN arguments take the library calls.
+template <bool INV>
+__device__ __forceinline__ double root64(double a, double& inv) {
+  const int hi = __double2hiint(a);
+  if ((unsigned)(hi - 0x07b00000) >= 0x78400000u) {  // outside [2^-900, inf)
+    if (INV) inv = rsqrt(a);
+    return sqrt(a);
+  }
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double g0 = a * y;
+  const double h0 = __hiloint2double(__double2hiint(y) - 0x00100000, __double2loint(y));
+  const double r0 = fma(-g0, h0, 0.5);
+  const double g1 = fma(g0, r0, g0);
+  const double h1 = fma(h0, r0, h0);
+  if (INV) {
+    const double h2 = fma(h1, fma(-g1, h1, 0.5), h1);
+    inv = __hiloint2double(__double2hiint(h2) + 0x00100000, __double2loint(h2));
+  }
+  return fma(fma(-g1, g1, a), h1, g1);
+}
+__device__ __forceinline__ double root64(double a) {
+  double unused;
+  return root64<false>(a, unused);
+}
+
+// The quintic's interval of s, t = (its upper end) - s in [0, 1] (0 past the
+// support), and the selection of a coefficient per interval.  On each
+// interval W and its derivatives are one polynomial in t: Horner's rule takes
+// 5 (W), 4 (W') or 3 (W'') FMAs where the truncated powers of
+// kernel_kernel_quintic_spline.F90 took about 14, with no cancellation
+// between powers (the coefficients are small whole numbers).
+struct Interval {
+  bool in1, in2;
+  double t;
+};
+__device__ __forceinline__ Interval quintic_interval(double s) {
+  Interval q;
+  const int hs = __double2hiint(s);
+  q.in1 = hs < 0x3ff00000;  // s < 1
+  q.in2 = hs < 0x40000000;  // s < 2
+  const int top = q.in1 ? 0x3ff00000 : (q.in2 ? 0x40000000 : 0x40080000);
+  const double t = __hiloint2double(top, 0) - s;
+  q.t = hs < 0x40080000 ? t : 0.0;  // s < 3
+  return q;
+}
+__device__ __forceinline__ double pick(const Interval& q, int c1, int c2, int c3) {
+  // constants with a zero low word, given by their high words
+  return __hiloint2double(q.in1 ? c1 : (q.in2 ? c2 : c3), 0);
+}
+// high words of the coefficients
+constexpr int kC0 = 0, kP1 = 0x3ff00000, kP5 = 0x40140000, kM5 = (int)0xc0140000,
+              kP10 = 0x40240000, kP20 = 0x40340000, kM20 = (int)0xc0340000, kM25 = (int)0xc0390000,
+              kP26 = 0x403a0000, kP30 = 0x403e0000, kP40 = 0x40440000, kM40 = (int)0xc0440000,
+              kP50 = 0x40490000, kM60 = (int)0xc04e0000, kM80 = (int)0xc0540000,
+              kP100 = 0x40590000, kP120 = 0x405e0000, kM200 = (int)0xc0690000,
+              kP240 = 0x406e0000;
+
+// (3-s)^5 - 6(2-s)^5 + 15(1-s)^5, truncated: t^5 | 1 + 5t + 10t^2 + 10t^3 +
+// 5t^4 - 5t^5 | 26 + 50t + 20t^2 - 20t^3 - 20t^4 + 10t^5 from the outer
+// interval inwards
+__device__ __forceinline__ double quintic_w(double s) {
+  const Interval q = quintic_interval(s);
+  double w = fma(pick(q, kP10, kM5, kP1), q.t, pick(q, kM20, kP5, kC0));
+  w = fma(w, q.t, pick(q, kM20, kP10, kC0));
+  w = fma(w, q.t, pick(q, kP20, kP10, kC0));
+  w = fma(w, q.t, pick(q, kP50, kP5, kC0));
+  return fma(w, q.t, pick(q, kP26, kP1, kC0));
+}
+// 5(3-s)^4 - 30(2-s)^4 + 75(1-s)^4: 5t^4 | 5 + 20t + 30t^2 + 20t^3 - 25t^4 |
+// 50 + 40t - 60t^2 - 80t^3 + 50t^4
+__device__ __forceinline__ double quintic_g(const Interval& q) {
+  double g = fma(pick(q, kP50, kM25, kP5), q.t, pick(q, kM80, kP20, kC0));
+  g = fma(g, q.t, pick(q, kM60, kP30, kC0));
+  g = fma(g, q.t, pick(q, kP40, kP20, kC0));
+  return fma(g, q.t, pick(q, kP50, kP5, kC0));
+}
+// -20(3-s)^3 + 120(2-s)^3 - 300(1-s)^3: -20t^3 | -20 - 60t - 60t^2 + 100t^3 |
+// -40 + 120t + 240t^2 - 200t^3
+__device__ __forceinline__ double quintic_g2(const Interval& q) {
+  double g = fma(pick(q, kM200, kP100, kM20), q.t, pick(q, kP240, kM60, kC0));
+  g = fma(g, q.t, pick(q, kP120, kM60, kC0));
+  return fma(g, q.t, pick(q, kM40, kM20, kC0));
+}
+
 // W(r): kernel_kernel_quintic_spline.F90:69-99 (h = rc/3, W = coef*[(3-s)^5
 // - 6(2-s)^5 + 15(1-s)^5] piecewise) and kernel_kernel_Lucy.F90:68-78.
 template <typename T>
 __device__ __forceinline__ T kernel_w(const Consts& k, T r) {
   const T s = KC<T>::arg(k, r);
   if (k.kernel_type == 1) {
+    if constexpr (std::is_same<T, double>::value) return KC<T>::coef(k) * quintic_w(s);
     const T s3 = T(3) - s, s2 = T(2) - s, s1 = T(1) - s;
     T a3 = s3 * s3;
     a3 = a3 * a3 * s3;
@@ -76,6 +202,8 @@ template <typename T>
 __device__ __forceinline__ T kernel_gradw(const Consts& k, T r) {
   const T s = KC<T>::arg(k, r);
   if (k.kernel_type == 1) {
+    if constexpr (std::is_same<T, double>::value)
+      return KC<T>::coef_grad(k) * quintic_g(quintic_interval(s));
     const T s3 = T(3) - s, s2 = T(2) - s, s1 = T(1) - s;
     T g = T(0);
     if (s < T(3)) {
@@ -125,6 +253,12 @@ __device__ __forceinline__ void kernel_gradw2(const Consts& k, T r, T& gw, T& g2
   const T s = r * KC<T>::inv_h(k);
   const T cgr = KC<T>::coef_grad(k);
   if (k.kernel_type == 1) {
+    if constexpr (std::is_same<T, double>::value) {
+      const Interval q = quintic_interval(s);
+      gw = cgr * quintic_g(q);
+      g2 = (cgr * KC<T>::inv_h(k)) * quintic_g2(q);
+      return;
+    }
     const T s3 = T(3) - s, s2 = T(2) - s, s1 = T(1) - s;
     T a = T(0), b = T(0);
     if (s < T(3)) {
@@ -209,10 +343,25 @@ __device__ __forceinline__ T boundary_A(int type, T p_fluid, T B) {
   }
 }
 
+// a normal of the pair's random term in the path's type
+template <typename T>
+__device__ __forceinline__ T normal_as(float z);
+template <>
+__device__ __forceinline__ double normal_as<double>(float z) { return widen(z); }
+template <>
+__device__ __forceinline__ float normal_as<float>(float z) { return z; }
+
+// a with the sign of s (+-1) applied
+__device__ __forceinline__ double oriented(double a, float s) {
+  return __hiloint2double(__double2hiint(a) ^ (int)(__float_as_uint(s) & 0x80000000u),
+                          __double2loint(a));
+}
+__device__ __forceinline__ float oriented(float a, float s) { return a * s; }
+
 template <typename T>
 __device__ __forceinline__ T my_sqrt(T a);
 template <>
-__device__ __forceinline__ double my_sqrt<double>(double a) { return sqrt(a); }
+__device__ __forceinline__ double my_sqrt<double>(double a) { return root64(a); }
 template <>
 __device__ __forceinline__ float my_sqrt<float>(float a) { return sqrtf(a); }
 
@@ -295,13 +444,16 @@ __device__ __forceinline__ void pair_force(const Consts& k, const T* r, T inv_d,
         // g (pair_draw), s = +-1 by pid order so both sides get opposite We
         const T cb = T(0.70710678118654752440);
         const T ca = (D == 3) ? T(0.81649658092772603273) : cb;  // sqrt(1 - 1/d)
+        T zt[3];
+#pragma unroll
+        for (int a = 0; a < D; ++a) zt[a] = normal_as<T>(z[a]);
         T eg = T(0);
 #pragma unroll
-        for (int a = 0; a < D; ++a) eg += e[a] * (T)z[a];
-        const T f_r = my_sqrt<T>(T(-4) * kt * f_d) * inv_sqdt * (T)z[5];
+        for (int a = 0; a < D; ++a) eg += e[a] * zt[a];
+        const T f_r = oriented(my_sqrt<T>(T(-4) * kt * f_d) * inv_sqdt, z[5]);
         const T fl = f_r * (ca - cb) * eg, ft = f_r * cb;
 #pragma unroll
-        for (int a = 0; a < D; ++a) g[a] += fl * e[a] + ft * (T)z[a];
+        for (int a = 0; a < D; ++a) g[a] += fl * e[a] + ft * zt[a];
       }
       break;
     }

@@ -1175,34 +1175,34 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
               }
             }
           }
-          // owner side (Kahan-compensated in FP32)
-          {
-            const unsigned peers = __match_any_sync(amask, ow_l);
-            T s0 = vis[0], s1 = vis[1], s2 = vis[2];
-            if (peers != (1u << lane)) {
-              s0 = s1 = s2 = T(0);
-              for (unsigned mm = peers; mm; mm &= mm - 1) {
-                const int src = __ffs(mm) - 1;
-                s0 += __shfl_sync(peers, vis[0], src);
-                s1 += __shfl_sync(peers, vis[1], src);
-                s2 += __shfl_sync(peers, vis[2], src);
-              }
-            }
-            if (lane == __ffs(peers) - 1) {
-              const T sv[3] = {s0, s1, s2};
+        }
+        // owner side: the round's lanes lie in owner order, so each owner's
+        // lanes are adjacent; five segmented shuffle steps leave the segment's
+        // sum in its first lane (15 FP64 adds a round in 3D; a loop over the
+        // segment's lanes took 96, half of the sweep's FP64 slots: 64^3 step
+        // 7.22 -> 5.21 ms)
 #pragma unroll
-              for (int a = 0; a < 3; ++a) {
-                T& acc = acc_s[a * 32 + ow_l];
-                if (FP64) {
-                  acc += sv[a];
-                } else {
-                  T& cmp = comp_s[a * 32 + ow_l];
-                  const T y = sv[a] - cmp;
-                  const T tt = acc + y;
-                  cmp = (tt - acc) - y;
-                  acc = tt;
-                }
-              }
+        for (int o = 1; o < 32; o <<= 1) {
+          const bool same = __shfl_down_sync(0xffffffffu, ow_l, o) == ow_l && lane + o < 32;
+#pragma unroll
+          for (int a = 0; a < D; ++a) {
+            const T t2 = __shfl_down_sync(0xffffffffu, vis[a], o);
+            if (same) vis[a] += t2;
+          }
+        }
+        const int ow_prev = __shfl_up_sync(0xffffffffu, ow_l, 1);
+        if (lane == 0 || ow_prev != ow_l) {
+#pragma unroll
+          for (int a = 0; a < D; ++a) {
+            T& acc = acc_s[a * 32 + ow_l];
+            if (FP64) {
+              acc += vis[a];
+            } else {
+              T& cmp = comp_s[a * 32 + ow_l];
+              const T y = vis[a] - cmp;
+              const T tt = acc + y;
+              cmp = (tt - acc) - y;
+              acc = tt;
             }
           }
         }

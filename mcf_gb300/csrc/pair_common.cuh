@@ -171,6 +171,28 @@ __device__ __forceinline__ double wrap_sep(double a, double b, double L) {
   return d;
 }
 
+// the components of a separation with an image (exact_sep)
+template <int D>
+__device__ __forceinline__ void image_sep(const Consts& k, const double* xi, const double* xj, int sh,
+                                       double* r) {
+#pragma unroll
+  for (int a = 0; a < D; ++a) {
+    const int s = (sh >> (2 * a)) & 3;
+    if (a == 0 && (sh & (kLeUp | kLeDown))) {
+      if (sh & kLeUp)
+        r[a] = wrap_sep(xi[0], f_modulo(__dadd_rn(xj[0], k.le_S), k.len[0]), k.len[0]);
+      else
+        r[a] = wrap_sep(f_modulo(__dadd_rn(xi[0], k.le_S), k.len[0]), xj[0], k.len[0]);
+    } else if (s == 1) {
+      r[a] = __dsub_rn(xi[a], __dadd_rn(xj[a], k.len[a]));
+    } else if (s == 2) {
+      r[a] = __dsub_rn(__dadd_rn(xi[a], k.len[a]), xj[a]);
+    } else {
+      r[a] = __dsub_rn(xi[a], xj[a]);
+    }
+  }
+}
+
 // FP64 separation of MCF's pair (ip, jp) where jp may be a periodic image:
 // PPM creates images only at x+L (symmetry=T), so a pair across a boundary
 // is evaluated as (x_upper) - (x_lower + L) per axis.  Rounded exactly like
@@ -184,26 +206,17 @@ __device__ __forceinline__ double wrap_sep(double a, double b, double L) {
 template <int D>
 __device__ __forceinline__ double exact_sep(const Consts& k, const double* xi, const double* xj,
                                             int sh, double* r) {
-  double d2 = 0.0;
+  // inside the box (most pairs) no image arithmetic is issued: as predicated
+  // code it took 6 of a pair's FP64 slots
+  if (sh == 0) {
 #pragma unroll
-  for (int a = 0; a < D; ++a) {
-    const int s = (sh >> (2 * a)) & 3;
-    double ra;
-    if (a == 0 && (sh & (kLeUp | kLeDown))) {
-      if (sh & kLeUp)
-        ra = wrap_sep(xi[0], f_modulo(__dadd_rn(xj[0], k.le_S), k.len[0]), k.len[0]);
-      else
-        ra = wrap_sep(f_modulo(__dadd_rn(xi[0], k.le_S), k.len[0]), xj[0], k.len[0]);
-    } else if (s == 1) {
-      ra = __dsub_rn(xi[a], __dadd_rn(xj[a], k.len[a]));
-    } else if (s == 2) {
-      ra = __dsub_rn(__dadd_rn(xi[a], k.len[a]), xj[a]);
-    } else {
-      ra = __dsub_rn(xi[a], xj[a]);
-    }
-    r[a] = ra;
-    d2 = (a == 0) ? __dmul_rn(ra, ra) : __dadd_rn(d2, __dmul_rn(ra, ra));
+    for (int a = 0; a < D; ++a) r[a] = __dsub_rn(xi[a], xj[a]);
+  } else {
+    image_sep<D>(k, xi, xj, sh, r);
   }
+  double d2 = __dmul_rn(r[0], r[0]);
+#pragma unroll
+  for (int a = 1; a < D; ++a) d2 = __dadd_rn(d2, __dmul_rn(r[a], r[a]));
   return d2;
 }
 

@@ -874,78 +874,67 @@ __global__ void __launch_bounds__(kReuseTPB, (NNW && D == 3) ? 4 : 5)
 }
 
 // ---------------------------------------------------------------------------
-// Symmetric force sweep: every pair is evaluated once, by the particle whose
-// cell owns it (partner in one of the 13 forward cells, or later in the same
-// cell: the half-shell of ppm_neighlist_MkNeighIdx.F90:198-249).  The owner
-// keeps its share in registers (Kahan in FP32); the partner's share is
-// summed per (forward slot, partner) in shared memory.  Lanes of a round that
-// hit the same partner are combined with __match_any_sync, in lane order,
-// by the lowest such lane, so every sum has a fixed order and the result is
-// deterministic without atomics.  The per-slot partial sums go to planes
-// jp[slot][c][n] that k_force_gather adds up per particle.
+// Symmetric FP64 force sweep: every pair is evaluated once, by the particle
+// whose cell owns it (partner in one of the 13 forward cells, or later in the
+// same cell: the half-shell of ppm_neighlist_MkNeighIdx.F90:198-249).  A warp
+// takes a cell; the owned pairs of its particles, in owner order, are dealt to
+// the lanes in runs of kRun consecutive pairs, so that all lanes work whatever
+// the particles' list lengths.  The partner's share is summed per (forward
+// slot, partner) in shared memory; lanes that hit the same partner in one
+// round are combined with __match_any_sync, in lane order, by the lowest such
+// lane.  The owner's share is summed in the lane while its run stays with one
+// owner, then over the lanes by a segmented shuffle.  Every sum has a fixed
+// order: the result is deterministic without atomics.  The partner sums go to
+// planes jp[slot][c][n] that k_force_gather adds up per particle.
+//
+// Bound: the FP64 pipe (84% busy); what counts is FP64 slots a pair.  Runs of
+// 4 spread the owner reduction (15 adds + 3) over 128 pairs; the mass factor
+// is left to the gather (not for the Morris form, whose factor is the
+// partner's mass).  64^3 with noise: 2.64 ms, 86 slots
+// a pair, against 3.02 ms and 100 with one pair a round and lane.
 // ---------------------------------------------------------------------------
-template <bool FP64>
-struct SymT;
-template <>
-struct SymT<true> {
-  using T = double;
-  static constexpr int CC = 32;  // partners per slot held in shared memory
-};
-template <>
-struct SymT<false> {
-  using T = float;
-  static constexpr int CC = 64;
-};
+constexpr int kSymCC = 32;  // partners per slot held in shared memory
+constexpr int kRun = 4;     // consecutive pairs a lane takes in a round
 
-
-// Per-warp dynamic shared memory of k_force_sym (bytes), see the layout in
-// the kernel.
-template <int D, bool FP64>
+// Per-warp dynamic shared memory of k_force_sym (bytes):
+// part[NSF][D][CC] | acc[D][32] | ex[33] e0[32] pad | x v pc [32] sid pid [32]
+template <int D>
 __host__ __device__ constexpr int sym_warp_bytes() {
-  using T = typename SymT<FP64>::T;
   constexpr int NSF = (D == 3) ? 14 : 5;
-  constexpr int CC = SymT<FP64>::CC;
-  constexpr int part = NSF * 3 * CC * (int)sizeof(T);
-  constexpr int accs = 2 * 3 * 32 * (int)sizeof(T);
-  constexpr int idx = 96 * 4;  // ex[33], e0[32], pad
-  constexpr int own = FP64 ? (3 * 32 * 32 + 2 * 32 * 4) : (3 * 32 * 16 + 32 * 8);
-  return ((part + accs + idx + own) + 31) / 32 * 32;
+  constexpr int part = NSF * D * kSymCC * 8;
+  constexpr int acc = D * 32 * 8;
+  constexpr int idx = 96 * 4;
+  constexpr int own = 3 * 32 * 32 + 2 * 32 * 4;
+  return (part + acc + idx + own + 31) / 32 * 32;
 }
 
-template <int D, bool FP64>
+template <int D>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     k_force_sym(Consts k, const int* __restrict__ cell_start, const uint16_t* __restrict__ nl,
                 const int* __restrict__ ncount, const int* __restrict__ nhs,
-                const float4* __restrict__ off, const double4_32a* __restrict__ x,
-                const double4_32a* __restrict__ v, const double4_32a* __restrict__ pc,
-                const float4* __restrict__ pcf, const float4* __restrict__ vf,
-                const float2* __restrict__ wd, const int* __restrict__ sid,
-                const int* __restrict__ pid, typename SymT<FP64>::T* __restrict__ jp,
-                uint32_t step_arg, const int64_t* __restrict__ step_ptr,
-                typename SymT<FP64>::T inv_sqdt) {
+                const double4_32a* __restrict__ x, const double4_32a* __restrict__ v,
+                const double4_32a* __restrict__ pc, const int* __restrict__ sid,
+                const int* __restrict__ pid, double* __restrict__ jp, uint32_t step_arg,
+                const int64_t* __restrict__ step_ptr, double inv_sqdt) {
   // the Philox counter's step: the argument, or the device step counter
   // when the sweep runs inside a captured graph
   const uint32_t step = step_ptr ? (uint32_t)*step_ptr : step_arg;
-  using T = typename SymT<FP64>::T;
-  constexpr int CC = SymT<FP64>::CC;
+  constexpr int CC = kSymCC;
   constexpr int CENTER = (D == 3) ? 13 : 4;
   constexpr int NSF = (D == 3) ? 14 : 5;  // forward slots CENTER..NS-1
   extern __shared__ __align__(32) unsigned char smem_raw[];
   __shared__ NbTable tab[kWarpsPerBlock];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // per-warp layout: part[NSF][3][CC] | acc[3][32] | comp[3][32] | ex[33] e0[32] |
-  //                  owner data (FP32: off, vf, pcf float4 + wd float2;
-  //                              FP64: x, v, pc double4 + sid, pid int)
-  unsigned char* wb = smem_raw + (size_t)wib * sym_warp_bytes<D, FP64>();
-  T* part = reinterpret_cast<T*>(wb);
-  T* acc_s = part + NSF * 3 * CC;
-  T* comp_s = acc_s + 3 * 32;
-  int* ex = reinterpret_cast<int*>(comp_s + 3 * 32);
+  unsigned char* wb = smem_raw + (size_t)wib * sym_warp_bytes<D>();
+  double* part = reinterpret_cast<double*>(wb);
+  double* acc_s = part + NSF * D * CC;
+  int* ex = reinterpret_cast<int*>(acc_s + D * 32);
   int* e0s = ex + 33;
-  unsigned char* own = reinterpret_cast<unsigned char*>(ex + 96);
+  double4_32a* ox = reinterpret_cast<double4_32a*>(ex + 96);
+  int* os = reinterpret_cast<int*>(ox + 96);
   const int n = k.n;
   const bool noise = k.noise != 0;
-  const bool walls = k.wall_axis != -1;
+  const bool scaled = k.rhs_force_type == 1;
   for (int cell = blockIdx.x * kWarpsPerBlock + wib; cell <= k.ncell;
        cell += gridDim.x * kWarpsPerBlock) {
     NbTable& t = tab[wib];
@@ -956,11 +945,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
       const int cs_ = t.count[CENTER + s], st_ = t.start[CENTER + s];
       for (int q = lane; q < cs_; q += 32)
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
+        for (int a = 0; a < D; ++a) {
           if (cs_ <= CC)
-            part[(s * 3 + a) * CC + q] = T(0);
+            part[(s * D + a) * CC + q] = 0.0;
           else
-            jp[((size_t)s * 3 + a) * n + st_ + q] = T(0);
+            jp[((size_t)s * D + a) * n + st_ + q] = 0.0;
         }
     }
     const int c0 = t.start[CENTER], c1 = c0 + t.count[CENTER];
@@ -970,38 +959,16 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
       const int e0 = act ? nhs[i] : 0, e1 = act ? ncount[i] : 0;
       const int len = e1 - e0;
       // owner data and accumulators of this chunk in shared memory
-      if (FP64) {
-        double4_32a* ox = reinterpret_cast<double4_32a*>(own);
-        double4_32a* ov = ox + 32;
-        double4_32a* oc = ov + 32;
-        int* os = reinterpret_cast<int*>(oc + 32);
-        int* op = os + 32;
-        if (act) {
-          ox[lane] = x[i];
-          ov[lane] = v[i];
-          oc[lane] = pc[i];
-          os[lane] = sid[i];
-          op[lane] = pid[i];
-        }
-      } else {
-        float4* oo = reinterpret_cast<float4*>(own);
-        float4* ov = oo + 32;
-        float4* oc = ov + 32;
-        float2* ow = reinterpret_cast<float2*>(oc + 32);
-        if (act) {
-          oo[lane] = off[i];
-          ov[lane] = vf[i];
-          oc[lane] = pcf[i];
-          if (walls && k.wall_axis >= 0) ow[lane] = wd[i];
-        }
+      if (act) {
+        ox[lane] = x[i];
+        ox[32 + lane] = v[i];
+        ox[64 + lane] = pc[i];
+        os[lane] = sid[i];
+        os[32 + lane] = pid[i];
       }
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        acc_s[a * 32 + lane] = T(0);
-        comp_s[a * 32 + lane] = T(0);
-      }
-      // exclusive prefix of the owned-pair counts: the warp's pairs are
-      // spread evenly over the lanes, 32 per round
+      for (int a = 0; a < D; ++a) acc_s[a * 32 + lane] = 0.0;
+      // exclusive prefix of the owned-pair counts
       int incl = len;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -1013,204 +980,147 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
       e0s[lane] = e0;
       if (lane == 31) ex[32] = total;
       __syncwarp();
-      const int rounds = (total + 31) >> 5;
-      for (int r = 0; r < rounds; ++r) {
-        const int fidx = r * 32 + lane;
-        const bool valid = fidx < total;
+      for (int r0 = 0; r0 < total; r0 += 32 * kRun) {
+        // the run's first pair and its owner
+        int fidx = r0 + lane * kRun;
         int ow_l = 0;
 #pragma unroll
         for (int stp = 16; stp > 0; stp >>= 1)
           if (ex[ow_l + stp] <= fidx) ow_l += stp;
-        bool has = false;
-        int keyj = 0, jsl = 0, jq = 0;
-        T vjs[3] = {0, 0, 0}, vis[3] = {0, 0, 0};
-        if (valid) {
-          const int ii = base + ow_l;
-          const int e = e0s[ow_l] + (fidx - ex[ow_l]);
-          const int ent = nl[(size_t)e * n + ii];
-          jsl = ent >> kLocalBits;
-          jq = ent & (kMaxCellCount - 1);
-          const int j = t.start[jsl] + jq;
-          T rr[3], vi[3], vj[3];
-          T Ai, Bi, Ci, Pi, Aj, Bj, Cj, Pj, inv_d, d;
-          int si, sj, pidi, pidj;
-          double xi[3] = {0.0, 0.0, 0.0}, xj[3] = {0.0, 0.0, 0.0};
-          float2 wdi = make_float2(0.f, 0.f);
-          if (FP64) {
-            const double4_32a* ox = reinterpret_cast<const double4_32a*>(own);
-            const int* os = reinterpret_cast<const int*>(ox + 96);
-            const double4_32a x4 = ox[ow_l], v4 = ox[32 + ow_l], c4 = ox[64 + ow_l];
-            si = os[ow_l];
-            pidi = os[32 + ow_l];
-            xi[0] = x4.x; xi[1] = x4.y; xi[2] = x4.z;
-            vi[0] = (T)v4.x; vi[1] = (T)v4.y; vi[2] = (T)v4.z;
-            Ai = (T)c4.x; Bi = (T)c4.y; Ci = (T)c4.z; Pi = (T)c4.w;
-            sj = sid[j];
-            const double4_32a xj4 = x[j];
-            xj[0] = xj4.x; xj[1] = xj4.y; xj[2] = xj4.z;
-            double r64[3];
-            const double d2 = exact_sep<D>(k, xi, xj, t.shift[jsl], r64);
+        double vis[3] = {0, 0, 0};  // the share of owner ow_l summed in this lane
+#pragma unroll 1
+        for (int u = 0; u < kRun; ++u, ++fidx) {
+          const bool valid = fidx < total;
+          // the run passes into the next owner's pairs: the finished owner's
+          // share goes to its sum (at most one lane ends a given owner's pairs)
+          const bool next = valid && fidx >= ex[ow_l + 1];
+          if (__any_sync(0xffffffffu, next)) {
+            if (next) {
 #pragma unroll
-            for (int a = 0; a < 3; ++a) rr[a] = (T)r64[a];
-            // MCF's correctly rounded SQRT for the kernel's argument (see
-            // k_force64)
-            double inv64;
-            d = (T)root64<true>(d2, inv64);
-            inv_d = (T)inv64;
-            const double4_32a vj4 = v[j], cj4 = pc[j];
-            vj[0] = (T)vj4.x; vj[1] = (T)vj4.y; vj[2] = (T)vj4.z;
-            Aj = (T)cj4.x; Bj = (T)cj4.y; Cj = (T)cj4.z; Pj = (T)cj4.w;
-            pidj = noise ? pid[j] : 0;
-          } else {
-            const float4* oo = reinterpret_cast<const float4*>(own);
-            const float2* ow = reinterpret_cast<const float2*>(oo + 96);
-            const float4 o4 = oo[ow_l], v4 = oo[32 + ow_l], c4 = oo[64 + ow_l];
-            si = __float_as_int(o4.w);
-            pidi = __float_as_int(v4.w);
-            vi[0] = (T)v4.x; vi[1] = (T)v4.y; vi[2] = (T)v4.z;
-            Ai = (T)c4.x; Bi = (T)c4.y; Ci = (T)c4.z; Pi = (T)c4.w;
-            if (walls && k.wall_axis >= 0) wdi = ow[ow_l];
-            const float4 oj = off[j], vj4 = vf[j], cj4 = pcf[j];
-            sj = __float_as_int(oj.w);
-            const float4 so = t.o[jsl];
-            rr[0] = (T)((o4.x - oj.x) - so.x);
-            rr[1] = (T)((o4.y - oj.y) - so.y);
-            rr[2] = (D == 3) ? (T)((o4.z - oj.z) - so.z) : T(0);
-            T d2 = rr[0] * rr[0] + rr[1] * rr[1];
-            if (D == 3) d2 += rr[2] * rr[2];
-            inv_d = (T)rsqrtf((float)d2);
-            d = d2 * inv_d;
-            vj[0] = (T)vj4.x; vj[1] = (T)vj4.y; vj[2] = (T)vj4.z;
-            Aj = (T)cj4.x; Bj = (T)cj4.y; Cj = (T)cj4.z; Pj = (T)cj4.w;
-            pidj = __float_as_int(vj4.w);
+              for (int a = 0; a < D; ++a) {
+                acc_s[a * 32 + ow_l] += vis[a];
+                vis[a] = 0.0;
+              }
+              do ++ow_l;
+              while (fidx >= ex[ow_l + 1]);
+            }
           }
-          has = !(si != 0 && sj != 0);  // w-w, c-c, c-w: no interaction here
-          if (has) {
-            if (si < 0 || sj < 0) {
-              // fluid-wall pair (pp_interaction_fw.inc / _wf.inc)
-              const int sw = (sj < 0) ? sj : si;
-              const int face = -sw;
-              const bool lower = (face & 1) != 0;
-              const int axis = (face - 1) >> 1;
-              T df, dw;
-              if (!FP64 && k.wall_axis >= 0) {
-                const float2 wj = wd[j];
-                const float a_ = lower ? wdi.x : wdi.y, b_ = lower ? wj.x : wj.y;
-                df = (T)((sj < 0) ? a_ : b_);
-                dw = (T)((sj < 0) ? b_ : a_);
-              } else {
-                const double x_sur = axis == 0 ? (lower ? k.min_phys[0] : k.max_phys[0])
-                                     : axis == 1 ? (lower ? k.min_phys[1] : k.max_phys[1])
-                                                 : (lower ? k.min_phys[2] : k.max_phys[2]);
-                double xa, xb;
-                if (FP64) {
-                  xa = axis == 0 ? xi[0] : axis == 1 ? xi[1] : xi[2];
-                  xb = axis == 0 ? xj[0] : axis == 1 ? xj[1] : xj[2];
+          bool has = false;
+          int keyj = 0, jsl = 0, jq = 0;
+          double g[3] = {0, 0, 0}, s_j = 1.0;
+          if (valid) {
+            const int ii = base + ow_l;
+            const int e = e0s[ow_l] + (fidx - ex[ow_l]);
+            const int ent = nl[(size_t)e * n + ii];
+            jsl = ent >> kLocalBits;
+            jq = ent & (kMaxCellCount - 1);
+            const int j = t.start[jsl] + jq;
+            const int si = os[ow_l], sj = sid[j];
+            has = !(si != 0 && sj != 0);  // w-w, c-c, c-w: no interaction here
+            if (has) {
+              const double4_32a x4 = ox[ow_l], v4 = ox[32 + ow_l], c4 = ox[64 + ow_l];
+              const double4_32a xj4 = x[j], vj4 = v[j], cj4 = pc[j];
+              const double xi[3] = {x4.x, x4.y, x4.z}, xj[3] = {xj4.x, xj4.y, xj4.z};
+              double rr[3] = {0, 0, 0};
+              const double d2 = exact_sep<D>(k, xi, xj, t.shift[jsl], rr);
+              // MCF's correctly rounded SQRT for the kernel's argument (see
+              // k_force64)
+              double inv_d;
+              const double d = root64<true>(d2, inv_d);
+              double vi[3] = {v4.x, v4.y, v4.z}, vj[3] = {vj4.x, vj4.y, vj4.z};
+              double Ai = c4.x, Aj = cj4.x;
+              if (si < 0 || sj < 0) {
+                // fluid-wall pair (pp_interaction_fw.inc / _wf.inc)
+                const int sw = (sj < 0) ? sj : si;
+                const int axis = (-sw - 1) >> 1;
+                const double xa = axis == 0 ? xi[0] : axis == 1 ? xi[1] : xi[2];
+                const double xb = axis == 0 ? xj[0] : axis == 1 ? xj[1] : xj[2];
+                double vw[3];
+                if (sj < 0) {
+                  wall_noslip<double, D>(k, xa, xb, vi, sj, vw);
+#pragma unroll
+                  for (int a = 0; a < D; ++a) vj[a] = vw[a];
+                  Aj = boundary_A<double>(k.rhs_force_type, c4.w, cj4.y);
                 } else {
-                  const double4_32a a4 = x[ii], b4 = x[j];
-                  xa = axis == 0 ? a4.x : axis == 1 ? a4.y : a4.z;
-                  xb = axis == 0 ? b4.x : axis == 1 ? b4.y : b4.z;
+                  wall_noslip<double, D>(k, xb, xa, vj, si, vw);
+#pragma unroll
+                  for (int a = 0; a < D; ++a) vi[a] = vw[a];
+                  Ai = boundary_A<double>(k.rhs_force_type, cj4.w, c4.y);
                 }
-                df = (T)(((sj < 0) ? xa : xb) - x_sur);
-                dw = (T)(((sj < 0) ? xb : xa) - x_sur);
               }
-              T vw[3];
-              if (sj < 0) {
-                wall_noslip_dist<T, D>(k, df, dw, vi, sj, vw);
+              const double gw = kernel_gradw<double>(k, d);
+              double vij[3];
 #pragma unroll
-                for (int a = 0; a < D; ++a) vj[a] = vw[a];
-                Aj = boundary_A<T>(k.rhs_force_type, Pi, Bj);
+              for (int a = 0; a < D; ++a) vij[a] = vi[a] - vj[a];
+              float z[6];
+              if (noise) pair_draw<D>(k.rhs_force_type, k.rk, step, os[32 + ow_l], pid[j], z);
+              pair_force<double, D>(k, rr, inv_d, vij, Ai, c4.y, Aj, cj4.y, gw, noise, z,
+                                    inv_sqdt, g);
+              if (scaled) {
+#pragma unroll
+                for (int a = 0; a < D; ++a) vis[a] += g[a] * cj4.z;
+                s_j = c4.z;
               } else {
-                wall_noslip_dist<T, D>(k, df, dw, vj, si, vw);
 #pragma unroll
-                for (int a = 0; a < D; ++a) vi[a] = vw[a];
-                Ai = boundary_A<T>(k.rhs_force_type, Pj, Bi);
+                for (int a = 0; a < D; ++a) vis[a] += g[a];
               }
+              keyj = (jsl - CENTER) * kMaxCellCount + jq;
             }
-            const T gw = kernel_gradw<T>(k, d);
-            T vij[3];
-#pragma unroll
-            for (int a = 0; a < D; ++a) vij[a] = vi[a] - vj[a];
-            float z[6];
-            if (noise) pair_draw<D>(k.rhs_force_type, k.rk, step, pidi, pidj, z);
-            T g[3], s_i, s_j;
-            pair_force<T, D>(k, rr, inv_d, vij, Ai, Bi, Aj, Bj, gw, noise, z, inv_sqdt, g);
-            pair_scales<T>(k.rhs_force_type, Ci, Cj, s_i, s_j);
-#pragma unroll
-            for (int a = 0; a < D; ++a) {
-              vis[a] = g[a] * s_i;
-              vjs[a] = -g[a] * s_j;
-            }
-            keyj = (jsl - CENTER) * kMaxCellCount + jq;
           }
-        }
-        // deterministic combination: lanes of this round with the same
-        // target are summed in lane order by the lowest of them
-        const unsigned amask = __ballot_sync(0xffffffffu, has);
-        if (has) {
-          // partner side
-          {
+          // partner side: lanes with the same partner are summed in lane
+          // order by the lowest of them
+          const unsigned amask = __ballot_sync(0xffffffffu, has);
+          if (has) {
+            if (scaled) {
+#pragma unroll
+              for (int a = 0; a < D; ++a) g[a] *= s_j;
+            }
             const unsigned peers = __match_any_sync(amask, keyj);
-            T s0 = vjs[0], s1 = vjs[1], s2 = vjs[2];
+            double sum[3] = {g[0], g[1], g[2]};
             if (peers != (1u << lane)) {
-              s0 = s1 = s2 = T(0);
+              sum[0] = sum[1] = sum[2] = 0.0;
               for (unsigned mm = peers; mm; mm &= mm - 1) {
                 const int src = __ffs(mm) - 1;
-                s0 += __shfl_sync(peers, vjs[0], src);
-                s1 += __shfl_sync(peers, vjs[1], src);
-                s2 += __shfl_sync(peers, vjs[2], src);
+#pragma unroll
+                for (int a = 0; a < D; ++a) sum[a] += __shfl_sync(peers, g[a], src);
               }
             }
             if (lane == __ffs(peers) - 1) {
               const int s = jsl - CENTER;
               if (t.count[jsl] <= CC) {
-                part[(s * 3 + 0) * CC + jq] += s0;
-                part[(s * 3 + 1) * CC + jq] += s1;
-                part[(s * 3 + 2) * CC + jq] += s2;
+#pragma unroll
+                for (int a = 0; a < D; ++a) part[(s * D + a) * CC + jq] -= sum[a];
               } else {
                 const size_t b0 = (size_t)t.start[jsl] + jq;
-                jp[((size_t)s * 3 + 0) * n + b0] += s0;
-                jp[((size_t)s * 3 + 1) * n + b0] += s1;
-                jp[((size_t)s * 3 + 2) * n + b0] += s2;
+#pragma unroll
+                for (int a = 0; a < D; ++a) jp[((size_t)s * D + a) * n + b0] -= sum[a];
               }
             }
           }
+          __syncwarp();
         }
-        // owner side: the round's lanes lie in owner order, so each owner's
-        // lanes are adjacent; five segmented shuffle steps leave the segment's
-        // sum in its first lane (15 FP64 adds a round in 3D; a loop over the
-        // segment's lanes took 96, half of the sweep's FP64 slots: 64^3 step
-        // 7.22 -> 5.21 ms)
+        // owner side: the runs lie in owner order, so the lanes whose run ends
+        // with one owner are adjacent; five segmented shuffle steps leave their
+        // sum in the first of them
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
           const bool same = __shfl_down_sync(0xffffffffu, ow_l, o) == ow_l && lane + o < 32;
 #pragma unroll
           for (int a = 0; a < D; ++a) {
-            const T t2 = __shfl_down_sync(0xffffffffu, vis[a], o);
+            const double t2 = __shfl_down_sync(0xffffffffu, vis[a], o);
             if (same) vis[a] += t2;
           }
         }
         const int ow_prev = __shfl_up_sync(0xffffffffu, ow_l, 1);
         if (lane == 0 || ow_prev != ow_l) {
 #pragma unroll
-          for (int a = 0; a < D; ++a) {
-            T& acc = acc_s[a * 32 + ow_l];
-            if (FP64) {
-              acc += vis[a];
-            } else {
-              T& cmp = comp_s[a * 32 + ow_l];
-              const T y = vis[a] - cmp;
-              const T tt = acc + y;
-              cmp = (tt - acc) - y;
-              acc = tt;
-            }
-          }
+          for (int a = 0; a < D; ++a) acc_s[a * 32 + ow_l] += vis[a];
         }
         __syncwarp();
       }
       if (act) {
 #pragma unroll
-        for (int a = 0; a < 3; ++a) jp[((size_t)NSF * 3 + a) * n + i] = acc_s[a * 32 + lane];
+        for (int a = 0; a < D; ++a) jp[((size_t)NSF * D + a) * n + i] = acc_s[a * 32 + lane];
       }
       __syncwarp();
     }
@@ -1220,23 +1130,24 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
       if (cs_ > CC) continue;
       for (int q = lane; q < cs_; q += 32)
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-          jp[((size_t)s * 3 + a) * n + st_ + q] = part[(s * 3 + a) * CC + q];
+        for (int a = 0; a < D; ++a)
+          jp[((size_t)s * D + a) * n + st_ + q] = part[(s * D + a) * CC + q];
     }
     __syncwarp();
   }
 }
 
 // Sum of the per-slot partner shares and the owner share of every particle
-// (fixed order, Kahan in FP32), then body force and the second half kick.
-template <int D, bool FP64>
+// (fixed order) times the mass factor, then body force and the second half
+// kick.
+template <int D>
 __global__ void k_force_gather(Consts k, const int* __restrict__ cell_of,
-                               const typename SymT<FP64>::T* __restrict__ jp,
+                               const double* __restrict__ jp,
                                const double4_32a* __restrict__ x,
-                               const double4_32a* __restrict__ v, const int* __restrict__ sid,
+                               const double4_32a* __restrict__ v,
+                               const double4_32a* __restrict__ pc, const int* __restrict__ sid,
                                double4_32a* __restrict__ f, int fuse_mode, double dt,
                                double4_32a* __restrict__ v_out, unsigned* __restrict__ err) {
-  using T = typename SymT<FP64>::T;
   constexpr int CENTER = (D == 3) ? 13 : 4;
   constexpr int NSF = (D == 3) ? 14 : 5;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1252,9 +1163,9 @@ __global__ void k_force_gather(Consts k, const int* __restrict__ cell_of,
       rem /= k.nm[a];
     }
   }
-  T acc[3], comp[3] = {0, 0, 0};
+  double acc[3] = {0, 0, 0};
 #pragma unroll
-  for (int a = 0; a < 3; ++a) acc[a] = jp[((size_t)NSF * 3 + a) * n + j];
+  for (int a = 0; a < D; ++a) acc[a] = jp[((size_t)NSF * D + a) * n + j];
   if (cj < k.ncell) {
 #pragma unroll
     for (int s = 0; s < NSF; ++s) {
@@ -1269,23 +1180,18 @@ __global__ void k_force_gather(Consts k, const int* __restrict__ cell_of,
       }
       if (!ok) continue;
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        const T val = jp[((size_t)s * 3 + a) * n + j];
-        if (FP64) {
-          acc[a] += val;
-        } else {
-          const T y = val - comp[a];
-          const T tt = acc[a] + y;
-          comp[a] = (tt - acc[a]) - y;
-          acc[a] = tt;
-        }
-      }
+      for (int a = 0; a < D; ++a) acc[a] += jp[((size_t)s * D + a) * n + j];
     }
+  }
+  if (k.rhs_force_type != 1) {
+    const double scale = pc[j].z;
+#pragma unroll
+    for (int a = 0; a < D; ++a) acc[a] *= scale;
   }
   const double4_32a x4 = x[j];
   const double xj[3] = {x4.x, x4.y, x4.z};
-  force_epilogue<D>(k, j, sid[j], xj, (double)acc[0], (double)acc[1],
-                    D == 3 ? (double)acc[2] : 0.0, fuse_mode, dt, v, f, v_out, err);
+  force_epilogue<D>(k, j, sid[j], xj, acc[0], acc[1], D == 3 ? acc[2] : 0.0, fuse_mode, dt, v, f,
+                    v_out, err);
 }
 
 static int grid_for(Handle* h) {
@@ -1396,29 +1302,21 @@ int compute_force(Handle* h, int64_t step, int fuse_mode, double dt) {
     // symmetric sweep's shared-memory partner sums cap its occupancy)
     const int n = (int)h->n;
     const int gbn = (n + 255) / 256;
-    // the attribute is per device: set it for the handle's (a host call)
-    if (k.d == 3)
-      cudaFuncSetAttribute(k_force_sym<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kWarpsPerBlock * sym_warp_bytes<3, true>());
-    else
-      cudaFuncSetAttribute(k_force_sym<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kWarpsPerBlock * sym_warp_bytes<2, true>());
     double* jp = (double*)h->jp;
-    if (k.d == 3) {
-      k_force_sym<3, true><<<g, bs, kWarpsPerBlock * sym_warp_bytes<3, true>(), s>>>(
-          k, h->cell_start, h->nl, h->ncount, h->nhs, h->off, h->x, h->v, h->pc, h->pcf, h->vf,
-          h->wd, h->sid, h->pid, jp, (uint32_t)step, step_ptr, inv_sqdt);
-      if (n > 0)
-        k_force_gather<3, true><<<gbn, 256, 0, s>>>(k, h->cell_of, jp, h->x, h->v, h->sid, h->f,
-                                                    fuse_mode, dt, h->v2, h->d_err);
-    } else {
-      k_force_sym<2, true><<<g, bs, kWarpsPerBlock * sym_warp_bytes<2, true>(), s>>>(
-          k, h->cell_start, h->nl, h->ncount, h->nhs, h->off, h->x, h->v, h->pc, h->pcf, h->vf,
-          h->wd, h->sid, h->pid, jp, (uint32_t)step, step_ptr, inv_sqdt);
-      if (n > 0)
-        k_force_gather<2, true><<<gbn, 256, 0, s>>>(k, h->cell_of, jp, h->x, h->v, h->sid, h->f,
-                                                    fuse_mode, dt, h->v2, h->d_err);
-    }
+    // the attribute is per device: set it for the handle's (a host call)
+#define LAUNCH_SYM(DD)                                                                           \
+  do {                                                                                           \
+    constexpr int bytes = kWarpsPerBlock * sym_warp_bytes<DD>();                                 \
+    cudaFuncSetAttribute(k_force_sym<DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);   \
+    k_force_sym<DD><<<g, bs, bytes, s>>>(k, h->cell_start, h->nl, h->ncount, h->nhs, h->x, h->v, \
+                                         h->pc, h->sid, h->pid, jp, (uint32_t)step, step_ptr,    \
+                                         inv_sqdt);                                              \
+    if (n > 0)                                                                                   \
+      k_force_gather<DD><<<gbn, 256, 0, s>>>(k, h->cell_of, jp, h->x, h->v, h->pc, h->sid, h->f, \
+                                             fuse_mode, dt, h->v2, h->d_err);                    \
+  } while (0)
+    if (k.d == 3) LAUNCH_SYM(3); else LAUNCH_SYM(2);
+#undef LAUNCH_SYM
     h->launches++;
   } else if (fp64) {
 #define LAUNCH_F64(DD, NW)                                                                      \

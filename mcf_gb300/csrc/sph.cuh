@@ -343,20 +343,11 @@ __device__ __forceinline__ T boundary_A(int type, T p_fluid, T B) {
   }
 }
 
-// a normal of the pair's random term in the path's type
-template <typename T>
-__device__ __forceinline__ T normal_as(float z);
-template <>
-__device__ __forceinline__ double normal_as<double>(float z) { return widen(z); }
-template <>
-__device__ __forceinline__ float normal_as<float>(float z) { return z; }
-
 // a with the sign of s (+-1) applied
 __device__ __forceinline__ double oriented(double a, float s) {
   return __hiloint2double(__double2hiint(a) ^ (int)(__float_as_uint(s) & 0x80000000u),
                           __double2loint(a));
 }
-__device__ __forceinline__ float oriented(float a, float s) { return a * s; }
 
 template <typename T>
 __device__ __forceinline__ T my_sqrt(T a);
@@ -433,6 +424,31 @@ __device__ __forceinline__ void pair_force(const Consts& k, const T* r, T inv_d,
       break;
     }
     case 3: {
+      if constexpr (std::is_same<T, double>::value) {
+        // the same force along r instead of e = r/d, the constants of the
+        // amplitude folded: fewer FP64 slots (27 against 35 with noise)
+        const double gwu = gw * inv_d;
+        const double f_d = (eta * gwu) * (Bi + Bj);
+        double along = -(gwu * (Ai + Aj));
+        if (noise) {
+          const double cb = 0.70710678118654752440;
+          const double cr = (D == 3) ? 0.81649658092772603273 / cb - 1.0 : 0.0;  // ca/cb - 1
+          double zt[3], rz = 0.0;
+#pragma unroll
+          for (int a = 0; a < D; ++a) zt[a] = widen(z[a]);
+#pragma unroll
+          for (int a = 0; a < D; ++a) rz += r[a] * zt[a];
+          // f_r cb = sqrt(-4 kT f_d cb^2 / dt)
+          const double ft = oriented(root64(f_d * (-2.0 * kt * inv_sqdt * inv_sqdt)), z[5]);
+          if (D == 3) along += ft * cr * (rz * inv_d) * inv_d;
+#pragma unroll
+          for (int a = 0; a < D; ++a) g[a] = f_d * vij[a] + along * r[a] + ft * zt[a];
+        } else {
+#pragma unroll
+          for (int a = 0; a < D; ++a) g[a] = f_d * vij[a] + along * r[a];
+        }
+        break;
+      }
       const T f_c = (Ai + Aj) * gw;
       const T f_d = eta * (Bi + Bj) * gw * inv_d;
 #pragma unroll
@@ -444,16 +460,13 @@ __device__ __forceinline__ void pair_force(const Consts& k, const T* r, T inv_d,
         // g (pair_draw), s = +-1 by pid order so both sides get opposite We
         const T cb = T(0.70710678118654752440);
         const T ca = (D == 3) ? T(0.81649658092772603273) : cb;  // sqrt(1 - 1/d)
-        T zt[3];
-#pragma unroll
-        for (int a = 0; a < D; ++a) zt[a] = normal_as<T>(z[a]);
         T eg = T(0);
 #pragma unroll
-        for (int a = 0; a < D; ++a) eg += e[a] * zt[a];
-        const T f_r = oriented(my_sqrt<T>(T(-4) * kt * f_d) * inv_sqdt, z[5]);
+        for (int a = 0; a < D; ++a) eg += e[a] * (T)z[a];
+        const T f_r = my_sqrt<T>(T(-4) * kt * f_d) * inv_sqdt * (T)z[5];
         const T fl = f_r * (ca - cb) * eg, ft = f_r * cb;
 #pragma unroll
-        for (int a = 0; a < D; ++a) g[a] += fl * e[a] + ft * zt[a];
+        for (int a = 0; a < D; ++a) g[a] += fl * e[a] + ft * (T)z[a];
       }
       break;
     }

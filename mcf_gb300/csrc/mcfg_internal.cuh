@@ -352,8 +352,8 @@ int verlet_build_gated(Handle* h);
 int compute_density(Handle* h, bool with_pressure, bool reuse = false);
 int compute_pressure(Handle* h);
 int compute_force(Handle* h, int64_t step, int fuse_mode, double dt);
-// FP32-mixed sweeps over the partitioned candidate list (sweep32.cu)
-int density_list(Handle* h, bool with_pressure);
+// FP32-mixed density over a partitioned candidate list (sweep32.cu)
+int density_list(Handle* h, bool with_pressure, const uint16_t* vl, const int* vcount, int vcap);
 int apply_body_force(Handle* h);
 int integrate_velocity(Handle* h, double dt, double lambda);
 int integrate_position(Handle* h, double dt);

@@ -1,24 +1,27 @@
-// pair_kernels.cu -- the two pair sweeps of the SDPD right-hand side.
+// pair_kernels.cu -- the pair sweeps of the SDPD right-hand side.
 //
-// Layout: particles sorted by cell (cell_list.cu).  One warp owns one cell
-// and walks its particles in chunks of 32 (lane = particle i).  The 27 (3D)
-// or 9 (2D) neighbour cells are resolved once per warp into a shared-memory
-// table (start, count, periodic image sign per axis).
+// Layout: particles sorted by cell (cell_list.cu).
 //
-// Sweep 1 (k_density): FP32 candidate test on cell offsets for every
-// particle of the neighbour cells (warp-uniform broadcast loads), appending
-// candidates to a per-particle neighbour list [capacity][N] of 16-bit
-// entries slot<<11 | local index (coalesced across lanes).  Phase 2 walks the
-// list: the FP64 path re-tests with the exact FP64 squared distance of MCF
-// (so the pair set is MCF's bit for bit) and keeps only pairs inside the
-// cut-off; both paths then sum W.  The epilogue evaluates the equation of
-// state and writes the per-particle pair coefficients.
+// Candidates (k_scan): one warp owns one cell and walks its particles in
+// chunks of 32 (lane = particle i) through the 27 (3D) or 9 (2D) neighbour
+// cells, an FP32 test on cell offsets; the hits go to a per-particle list
+// [capacity][N] of 16-bit entries slot<<11 | local index (coalesced across
+// lanes).  With list reuse the list holds the candidates within rc + skin and
+// outlives the step, otherwise it is made for this step.
 //
-// Sweep 2 (k_force): walks the neighbour list (no candidate tests, no
-// divergence beyond list-length differences) and gathers the pair
+// Density (k_density_reuse here for FP64, k_density_list in sweep32.cu for
+// FP32-mixed): thread per particle (several lanes each on small systems) over
+// the candidates.  The FP64 path re-tests them with the exact FP64 squared
+// distance of MCF (so the pair set is MCF's bit for bit); both paths keep the
+// step's pairs as the list of the force sweep and sum W.  The epilogue
+// evaluates the equation of state and writes the per-particle pair
+// coefficients.
+//
+// Force (k_force32, k_force64): walks the step's list and gathers the pair
 // accelerations of particle i.  Each pair is evaluated from both sides, so
 // there is no scatter, no atomic and the result is deterministic; the random
 // term is keyed by the unordered pid pair, so both sides draw the same dW.
+// k_force_sym evaluates each pair once (FP64 Newtonian without stress).
 //
 // Reference: particles_compute_density.F90:369-867, particles_compute_
 // interaction.F90:609-900, pp_interaction*.inc, rhs_force_ff_Newtonian*.F90.
@@ -26,192 +29,48 @@
 #include <type_traits>
 
 #include "mcfg_internal.cuh"
+#include "packed.cuh"
 #include "pair_common.cuh"
 #include "sph.cuh"
 #include "sweep_common.cuh"
 
 namespace mcfg {
 
-constexpr int kStage = 64;      // neighbour-cell offsets staged per pass
-constexpr int kListStage = 96;  // neighbour entries staged in shared memory per lane
+constexpr int kMaskRows = 32;  // candidate chunks a warp notes between two emissions
 
-template <int D, bool FP64>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-    k_density(Consts k, const int* __restrict__ cell_start, const float4* __restrict__ off,
-              const double4_32a* __restrict__ x, const double4_32a* __restrict__ v,
-              const double* __restrict__ m, const int* __restrict__ sid,
-              const int* __restrict__ pid, uint16_t* __restrict__ nl, int* __restrict__ ncount,
-              int* __restrict__ nhs, int cap, double* __restrict__ rho, double* __restrict__ pr,
-              double4_32a* __restrict__ pc, float4* __restrict__ pcf, float4* __restrict__ vf,
-              int with_pressure, unsigned* __restrict__ err, int* __restrict__ stats,
-              unsigned long long* __restrict__ pairs, NN nn, CollArgs ca) {
-  constexpr int CENTER = (D == 3) ? 13 : 4;
-  __shared__ NbTable tab[kWarpsPerBlock];
-  __shared__ float4 sb[kWarpsPerBlock][kStage];
-  __shared__ uint16_t ls[kWarpsPerBlock][kListStage][32];
-  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = k.n;
-  int my_max = 0;
-  unsigned long long my_pairs = 0;
-  for (int cell = blockIdx.x * kWarpsPerBlock + wib; cell <= k.ncell;
-       cell += gridDim.x * kWarpsPerBlock) {
-    NbTable& t = tab[wib];
-    build_table<D>(k, cell, cell_start, t);
-    const int c0 = t.start[CENTER], c1 = c0 + t.count[CENTER];
-    for (int base = c0; base < c1; base += 32) {
-      const int i = base + lane;
-      const bool active = i < c1;
-      const float4 oi = active ? off[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float rlim = FP64 ? k.rc2f_hi : k.rc2f;
-      int cnt = 0;
-      // phase 1: candidate scan, offsets of each neighbour cell staged in
-      // shared memory by coalesced loads, then broadcast to the lanes
-      for (int sl = 0; sl < k.ns; ++sl) {
-        const int js = t.start[sl], jn = t.count[sl];
-        const float4 so = t.o[sl];
-        const float px = oi.x - so.x, py = oi.y - so.y, pz = oi.z - so.z;
-        for (int b2 = 0; b2 < jn; b2 += kStage) {
-          const int mm = min(kStage, jn - b2);
-          __syncwarp();
-          for (int q = lane; q < mm; q += 32) sb[wib][q] = off[js + b2 + q];
-          __syncwarp();
-#pragma unroll 4
-          for (int q2 = 0; q2 < mm; ++q2) {
-            const float4 oj = sb[wib][q2];
-            const float rx = px - oj.x, ry = py - oj.y;
-            float d2 = rx * rx + ry * ry;
-            if (D == 3) {
-              const float rz = pz - oj.z;
-              d2 += rz * rz;
-            }
-            const int q = b2 + q2;
-            if (active && d2 < rlim && !(sl == CENTER && js + q == i)) {
-              const uint16_t ent = (uint16_t)((sl << kLocalBits) | q);
-              if (cnt < kListStage)
-                ls[wib][cnt][lane] = ent;
-              else if (cnt < cap)
-                nl[(size_t)cnt * n + i] = ent;
-              ++cnt;
-            }
-          }
-        }
-      }
-      if (active && cnt > cap) {
-        atomicOr(err, kErrNeighOverflow);
-        my_max = max(my_max, cnt);
-      }
-      cnt = min(cnt, cap);
-      // phase 2: exact test (FP64 path), density sum, final list rows
-      const int si = active ? sid[i] : 0;
-      const bool acc_i = dyn_rho(k, si);
-      const int li = i - c0;  // local index in the cell
-      double rho_i = 0.0;
-      int kept = 0;
-      int hs = -1;  // first entry of the forward half (pairs this particle owns)
-      if (FP64) {
-        double4_32a xi4 = active ? x[i] : make_double4_32a(0, 0, 0, 0);
-        const double xi[3] = {xi4.x, xi4.y, xi4.z};
-        double sum = 0.0;
-        for (int e = 0; e < cnt; ++e) {
-          const int ent = (e < kListStage) ? ls[wib][e][lane] : nl[(size_t)e * n + i];
-          const int sl = ent >> kLocalBits, q = ent & (kMaxCellCount - 1);
-          const int j = t.start[sl] + q;
-          const double4_32a xj4 = x[j];
-          const double xj[3] = {xj4.x, xj4.y, xj4.z};
-          double r[3];
-          const double d2 = exact_sep<D>(k, xi, xj, t.shift[sl], r);
-          if (beyond(d2, k.rc2)) continue;
-          if (hs < 0 && (sl > CENTER || (sl == CENTER && q > li))) hs = kept;
-          nl[(size_t)kept * n + i] = (uint16_t)ent;
-          ++kept;
-          if (acc_i) {
-            const double w = kernel_w<double>(k, root64(d2));
-            sum += (k.rhs_density_type == 1) ? w * m[j] : w;
-          }
-        }
-        rho_i = sum;
-      } else {
-        // Kahan-compensated FP32 sum of W
-        float sum = 0.0f, comp = 0.0f;
-        const bool mass = k.rhs_density_type == 1;
-        for (int e = 0; e < cnt; ++e) {
-          const int ent = (e < kListStage) ? ls[wib][e][lane] : nl[(size_t)e * n + i];
-          if (e < kListStage) nl[(size_t)e * n + i] = (uint16_t)ent;
-          const int sl = ent >> kLocalBits, q = ent & (kMaxCellCount - 1);
-          if (hs < 0 && (sl > CENTER || (sl == CENTER && q > li))) hs = e;
-          if (!acc_i) continue;
-          const int j = t.start[sl] + q;
-          const float4 oj = off[j];
-          const float4 so = t.o[sl];
-          const float rx = (oi.x - oj.x) - so.x;
-          const float ry = (oi.y - oj.y) - so.y;
-          float d2 = rx * rx + ry * ry;
-          if (D == 3) {
-            const float rz = (oi.z - oj.z) - so.z;
-            d2 += rz * rz;
-          }
-          float w = kernel_w<float>(k, sqrtf(d2));
-          if (mass) w *= (float)m[j];
-          const float y = w - comp;
-          const float tt = sum + y;
-          comp = (tt - sum) - y;
-          sum = tt;
-        }
-        kept = cnt;
-        rho_i = (double)sum;
-      }
-      if (!active) continue;
-      ncount[i] = kept;
-      nhs[i] = (hs < 0) ? kept : hs;
-      my_max = max(my_max, kept);
-      my_pairs += (unsigned long long)kept;
-      const double mi = m[i];
-      double rho_out;
-      if (acc_i) {
-        rho_out = ((k.rhs_density_type == 1) ? k.w0 * mi : k.w0) + rho_i;
-      } else {
-        rho_out = (k.rhs_density_type == 1) ? k.init_density : k.init_density / mi;
-      }
-      rho[i] = rho_out;
-      if (!(rho_out > 0.0)) atomicOr(err, kErrZeroDensity);
-      if (with_pressure) {
-        const double4_32a vi4 =
-            (si > 0 && k.ncoll > 0) ? colloid_particle_update<D>(k, i, si, x[i], ca) : v[i];
-        write_particle_records<FP64>(k, i, rho_out, mi, pid[i], vi4, pr, pc, pcf, vf, nn);
-      }
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    my_max = max(my_max, __shfl_xor_sync(0xffffffffu, my_max, o));
-    my_pairs += __shfl_xor_sync(0xffffffffu, my_pairs, o);
-  }
-  if (lane == 0) {
-    atomicMax(&stats[1], my_max);
-    atomicAdd(pairs, my_pairs);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// List-reuse mode: the candidate list (gated rebuild) and the density sweep
-// over it.
-// ---------------------------------------------------------------------------
-
-// Candidates within rc + skin of every particle: k_density's FP32 scan of
-// the 27/9 neighbour cells with the larger bound, written to vl.  Returns at
-// once unless a rebuild is due.
+// Candidates of every particle with FP32 squared distance below lim, in slot
+// order and particle order, into list ([cap][n] rows) and count.  With
+// partition (FP32 lists) the fluid-fluid candidates fill the rows from 0 up,
+// the others from the last row down, and count = fluid-fluid | other << 16.
+// gate: return at once when *gate is zero (no rebuild due).
+//
+// Bound: instruction issue (a 3D particle meets 27 cells of ~28 particles, of
+// which ~113 are pairs).  So a chunk of 32 candidates is staged once in shared
+// memory as separate coordinates, tested two at a time by packed FP32
+// arithmetic against broadcast loads, and leaves one hit bit a candidate (the
+// sign of d2 - lim, shifted in): ~6 instructions a test with nothing done a
+// hit.  The bits are expanded afterwards, lanes near the same list row, so the
+// 2-byte stores coalesce (expanding chunk by chunk takes fewer instructions
+// but scatters them: 270 us).  The next chunk is in flight meanwhile.
+// 261,568 particles: 196 us (tests 113, expansion 83) where writing each hit
+// as it was found took 344 us.
 template <int D>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-    k_verlet_build(Consts k, const int* __restrict__ gate, const int* __restrict__ cell_start,
-                   const float4* __restrict__ off, uint16_t* __restrict__ vl,
-                   int* __restrict__ vcount, int vcap, int partition,
-                   unsigned* __restrict__ err) {
-  if (*gate == 0) return;
+    k_scan(Consts k, const int* __restrict__ gate, const int* __restrict__ cell_start,
+           const float4* __restrict__ off, float lim, uint16_t* __restrict__ list,
+           int* __restrict__ count, int cap, int partition, unsigned* __restrict__ err,
+           int* __restrict__ stats) {
+  if (gate && *gate == 0) return;
   constexpr int CENTER = (D == 3) ? 13 : 4;
+  constexpr float kFar = 3e18f;  // padding: far from everything, its square finite
   __shared__ NbTable tab[kWarpsPerBlock];
-  __shared__ float4 sb[kWarpsPerBlock][kStage];
+  __shared__ __align__(16) float sb[kWarpsPerBlock][2][3][32];
+  __shared__ unsigned s_mask[kWarpsPerBlock][kMaskRows][32];
+  __shared__ unsigned s_fluid[kWarpsPerBlock][kMaskRows];
+  __shared__ int s_ent[kWarpsPerBlock][kMaskRows];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = k.n;
+  const int n = k.n, ns = k.ns;
+  const F2 neg_lim = splat2(-lim);
   for (int cell = blockIdx.x * kWarpsPerBlock + wib; cell <= k.ncell;
        cell += gridDim.x * kWarpsPerBlock) {
     NbTable& t = tab[wib];
@@ -223,47 +82,124 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
       const float4 oi = active ? off[i] : make_float4(0.f, 0.f, 0.f, 0.f);
       const bool fluid_i = __float_as_int(oi.w) == 0;
       int cnt = 0, cnt_o = 0;  // cnt_o: partitioned lists' second segment
-      for (int sl = 0; sl < k.ns; ++sl) {
-        const int js = t.start[sl], jn = t.count[sl];
-        const float4 so = t.o[sl];
-        const float px = oi.x - so.x, py = oi.y - so.y, pz = oi.z - so.z;
-        for (int b2 = 0; b2 < jn; b2 += kStage) {
-          const int mm = min(kStage, jn - b2);
+      int rows = 0, buf = 0;
+      // one segment only: no partition, or all particles met are fluid
+      const bool plain0 = !partition || __all_sync(0xffffffffu, fluid_i);
+      bool plain = plain0;
+      // entries hold 11 bits of local index: a fuller cell is an error
+      // already (k_cell_finalize), and only its first 2048 are listed
+      int sl = 0, b2 = 0, jn = min(t.count[0], kMaxCellCount);
+      while (sl < ns && b2 >= jn) {
+        b2 = 0;
+        if (++sl < ns) jn = min(t.count[sl], kMaxCellCount);
+      }
+      const float4 pad = make_float4(kFar, kFar, kFar, 0.f);
+      float4 nx = (sl < ns && b2 + lane < jn) ? off[t.start[sl] + b2 + lane] : pad;
+      while (sl < ns) {
+        const int sl_c = sl, b_c = b2, mm = min(32, jn - b2);
+        float(*sc)[32] = sb[wib][buf];
+        sc[0][lane] = -nx.x;
+        sc[1][lane] = -nx.y;
+        if (D == 3) sc[2][lane] = -nx.z;
+        const unsigned fluid_j = __ballot_sync(0xffffffffu, __float_as_int(nx.w) == 0);
+        // the next chunk's offsets, in flight during this one's tests
+        b2 += 32;
+        while (sl < ns && b2 >= jn) {
+          b2 = 0;
+          if (++sl < ns) jn = min(t.count[sl], kMaxCellCount);
+        }
+        __syncwarp();
+        nx = (sl < ns && b2 + lane < jn) ? off[t.start[sl] + b2 + lane] : pad;
+        const float4 so = t.o[sl_c];
+        const F2 px = splat2(oi.x - so.x), py = splat2(oi.y - so.y), pz = splat2(oi.z - so.z);
+        unsigned mask = 0;
+        int q = 0;
+        for (; q < mm; q += 4) {
+          const ulonglong2 x4 = *reinterpret_cast<const ulonglong2*>(&sc[0][q]);
+          const ulonglong2 y4 = *reinterpret_cast<const ulonglong2*>(&sc[1][q]);
+          const F2 xa = add2(px, F2{x4.x}), xb = add2(px, F2{x4.y});
+          const F2 ya = add2(py, F2{y4.x}), yb = add2(py, F2{y4.y});
+          F2 da = fma2(ya, ya, mul2(xa, xa)), db = fma2(yb, yb, mul2(xb, xb));
+          if (D == 3) {
+            const ulonglong2 z4 = *reinterpret_cast<const ulonglong2*>(&sc[2][q]);
+            const F2 za = add2(pz, F2{z4.x}), zb = add2(pz, F2{z4.y});
+            da = fma2(za, za, da);
+            db = fma2(zb, zb, db);
+          }
+          float d0, d1, d2, d3;
+          unpack2(add2(da, neg_lim), d0, d1);
+          unpack2(add2(db, neg_lim), d2, d3);
+          mask = __funnelshift_l(__float_as_uint(d0), mask, 1);
+          mask = __funnelshift_l(__float_as_uint(d1), mask, 1);
+          mask = __funnelshift_l(__float_as_uint(d2), mask, 1);
+          mask = __funnelshift_l(__float_as_uint(d3), mask, 1);
+        }
+        // candidate c of the chunk at bit 31 - c
+        mask <<= 32 - q;
+        if (sl_c == CENTER) {
+          const int self = i - t.start[CENTER] - b_c;
+          if (self >= 0 && self < 32) mask &= ~(0x80000000u >> self);
+        }
+        if (!active) mask = 0;
+        if (__any_sync(0xffffffffu, mask != 0)) {
+          s_mask[wib][rows][lane] = mask;
+          if (lane == 0) {
+            s_ent[wib][rows] = (sl_c << kLocalBits) | b_c;
+            s_fluid[wib][rows] = __brev(fluid_j);
+          }
+          if (partition) plain = plain && fluid_j == 0xffffffffu;
+          ++rows;
+        }
+        buf ^= 1;
+        if (rows == kMaskRows || sl >= ns) {
+          // expand the bits, each lane its own rows in order
           __syncwarp();
-          for (int q = lane; q < mm; q += 32) sb[wib][q] = off[js + b2 + q];
-          __syncwarp();
-#pragma unroll 4
-          for (int q2 = 0; q2 < mm; ++q2) {
-            const float4 oj = sb[wib][q2];
-            const float rx = px - oj.x, ry = py - oj.y;
-            float d2 = rx * rx + ry * ry;
-            if (D == 3) {
-              const float rz = pz - oj.z;
-              d2 += rz * rz;
-            }
-            const int q = b2 + q2;
-            if (active && d2 < k.rv2f && !(sl == CENTER && js + q == i)) {
-              const uint16_t ent = (uint16_t)((sl << kLocalBits) | q);
-              if (partition && !(fluid_i && __float_as_int(oj.w) == 0)) {
-                // FP32 lists: pairs with a boundary particle from the last row down
-                if (cnt + cnt_o < vcap) vl[(size_t)(vcap - 1 - cnt_o) * n + i] = ent;
-                ++cnt_o;
-              } else {
-                if (cnt + cnt_o < vcap) vl[(size_t)cnt * n + i] = ent;
-                ++cnt;
+          int r = -1, ent0 = 0, left = cap - cnt - cnt_o;
+          unsigned m = 0;
+          if (plain) {
+            const int before = left;
+            uint16_t* dst = list + (size_t)cnt * n + i;
+            for (;;) {
+              while (m == 0 && r + 1 < rows) {
+                ++r;
+                m = s_mask[wib][r][lane];
+                ent0 = s_ent[wib][r];
               }
+              if (m == 0) break;
+              const int c = __clz(m);
+              m ^= 0x80000000u >> c;
+              if (left > 0) *dst = (uint16_t)(ent0 + c);
+              dst += n;
+              --left;
+            }
+            cnt += before - left;
+          } else {
+            for (;;) {
+              while (m == 0 && r + 1 < rows) m = s_mask[wib][++r][lane];
+              if (m == 0) break;
+              const int c = __clz(m);
+              m ^= 0x80000000u >> c;
+              const bool ff = fluid_i && ((s_fluid[wib][r] << c) >> 31);
+              if (left > 0)
+                list[(size_t)(ff ? cnt : cap - 1 - cnt_o) * n + i] = (uint16_t)(s_ent[wib][r] + c);
+              cnt += ff ? 1 : 0;
+              cnt_o += ff ? 0 : 1;
+              --left;
             }
           }
+          plain = plain0;
+          __syncwarp();
+          rows = 0;
         }
       }
       if (active) {
-        if (cnt + cnt_o > vcap) {
+        if (cnt + cnt_o > cap) {
           atomicOr(err, kErrNeighOverflow);
-          cnt = min(cnt, vcap);
-          cnt_o = min(cnt_o, vcap - cnt);
+          atomicMax(&stats[1], cnt + cnt_o);
+          cnt = min(cnt, cap);
+          cnt_o = min(cnt_o, cap - cnt);
         }
-        // partitioned: fluid-fluid count | other count << 16
-        vcount[i] = partition ? (cnt | (cnt_o << 16)) : cnt;
+        count[i] = partition ? (cnt | (cnt_o << 16)) : cnt;
       }
     }
   }
@@ -275,19 +211,25 @@ __global__ void k_rebuild_done(int* __restrict__ flag) {
   flag[0] = 0;
 }
 
-// FP64 density over the candidate list, one thread per particle: the step's
-// exact pair test with MCF's FP64 separation, the step's neighbour list for
-// the force sweeps (nhs: the first entry of the forward half the symmetric
-// sweep owns), the W sum and the epilogue of k_density.  The FP32 path runs
-// k_density_list (sweep32.cu).
-template <int D>
+// FP64 density over the candidate list: the step's exact pair test with
+// MCF's FP64 separation, the step's neighbour list for the force sweeps (nhs:
+// the first entry of the forward half the symmetric sweep owns), the W sum and
+// the per-particle epilogue.  vl and nl may be the same list (a step's own
+// candidates, compacted in place: a kept entry never lands behind one still
+// to be read).  The FP32 path runs k_density_list (sweep32.cu).
+//
+// S lanes per particle: the FP64 pipe needs about three warps per scheduler
+// (~58k threads) to stay busy, so small systems deal each particle's
+// candidates to 4 or 8 lanes; the lanes' sums are added in lane order.
+// 4,096 particles in 2D: 19 us with 8 lanes (one warp a cell, the lanes its
+// particles, took 50 us).
+template <int D, int S>
 __global__ void __launch_bounds__(kReuseTPB)
     k_density_reuse(Consts k, const int* __restrict__ cell_start, const int* __restrict__ cell_of,
                     const double4_32a* __restrict__ x, const double4_32a* __restrict__ v,
                     const double* __restrict__ m, const int* __restrict__ sid,
-                    const int* __restrict__ pid, const uint16_t* __restrict__ vl,
-                    const int* __restrict__ vcount, uint16_t* __restrict__ nl,
-                    int* __restrict__ ncount, int* __restrict__ nhs, int cap,
+                    const int* __restrict__ pid, const uint16_t* vl, const int* vcount,
+                    uint16_t* nl, int* ncount, int* __restrict__ nhs, int cap,
                     double* __restrict__ rho, double* __restrict__ pr,
                     double4_32a* __restrict__ pc, float4* __restrict__ pcf,
                     float4* __restrict__ vf, int with_pressure, unsigned* __restrict__ err,
@@ -297,7 +239,8 @@ __global__ void __launch_bounds__(kReuseTPB)
   __shared__ int s_start[kMaxStencil * kReuseTPB];
   __shared__ int s_shift[kMaxStencil * kReuseTPB];
   const int n = k.n, tid = threadIdx.x;
-  const int i = blockIdx.x * kReuseTPB + tid;
+  const int gt = blockIdx.x * kReuseTPB + tid;
+  const int i = gt / S, lane_s = gt % S;
   int my_max = 0;
   unsigned long long my_pairs = 0;
   if (i < n) {
@@ -309,44 +252,71 @@ __global__ void __launch_bounds__(kReuseTPB)
     const int cnt = vcount[i];
     const double4_32a xi4 = x[i];
     const double xi[3] = {xi4.x, xi4.y, xi4.z};
+    const int gbase = (tid & 31) & ~(S - 1);
+    const unsigned gmask = (S == 32 ? 0xffffffffu : (1u << S) - 1u) << gbase;
     double sum = 0.0;
-    int kept = 0, hs = -1;
-    for (int e = 0; e < cnt; ++e) {
-      const int ent = vl[(size_t)e * n + i];
-      const int sl = ent >> kLocalBits, q = ent & (kMaxCellCount - 1);
-      const int j = s_start[sl * kReuseTPB + tid] + q;
-      const double4_32a xj4 = x[j];
-      const double xj[3] = {xj4.x, xj4.y, xj4.z};
-      double r[3];
-      const double d2 = exact_sep<D>(k, xi, xj, s_shift[sl * kReuseTPB + tid], r);
-      if (beyond(d2, k.rc2)) continue;
-      if (hs < 0 && (sl > CENTER || (sl == CENTER && q > li))) hs = kept;
-      if (kept < cap) nl[(size_t)kept * n + i] = (uint16_t)ent;
-      ++kept;
-      if (acc_i) {
-        const double w = kernel_w<double>(k, root64(d2));
-        sum += (k.rhs_density_type == 1) ? w * m[j] : w;
+    int kept = 0, back = 0;  // back: kept entries before the forward half
+    for (int e0 = 0; e0 < cnt; e0 += S) {
+      const int e = e0 + lane_s;
+      bool in = false, fwd = false;
+      int ent = 0;
+      if (S == 1 || e < cnt) {
+        ent = vl[(size_t)e * n + i];
+        const int sl = ent >> kLocalBits, q = ent & (kMaxCellCount - 1);
+        const int j = s_start[sl * kReuseTPB + tid] + q;
+        const double4_32a xj4 = x[j];
+        const double xj[3] = {xj4.x, xj4.y, xj4.z};
+        double r[3];
+        const double d2 = exact_sep<D>(k, xi, xj, s_shift[sl * kReuseTPB + tid], r);
+        in = !beyond(d2, k.rc2);
+        fwd = sl > CENTER || (sl == CENTER && q > li);
+        if (in && acc_i) {
+          const double w = kernel_w<double>(k, root64(d2));
+          sum += (k.rhs_density_type == 1) ? w * m[j] : w;
+        }
+      }
+      if (S == 1) {
+        if (!in) continue;
+        if (kept < cap) nl[(size_t)kept * n + i] = (uint16_t)ent;
+        ++kept;
+        back += fwd ? 0 : 1;
+      } else {
+        // the group's ballots place the kept entries in candidate order
+        const unsigned bi = (__ballot_sync(gmask, in) & gmask) >> gbase;
+        const unsigned bf = (__ballot_sync(gmask, in && !fwd) & gmask) >> gbase;
+        const int pos = kept + __popc(bi & ((1u << lane_s) - 1u));
+        if (in && pos < cap) nl[(size_t)pos * n + i] = (uint16_t)ent;
+        kept += __popc(bi);
+        back += __popc(bf);
       }
     }
-    if (kept > cap) atomicOr(err, kErrNeighOverflow);
-    my_max = kept;
-    kept = min(kept, cap);
-    ncount[i] = kept;
-    nhs[i] = (hs < 0 || hs > kept) ? kept : hs;
-    my_pairs = (unsigned long long)kept;
-    const double mi = m[i];
-    double rho_out;
-    if (acc_i) {
-      rho_out = ((k.rhs_density_type == 1) ? k.w0 * mi : k.w0) + sum;
-    } else {
-      rho_out = (k.rhs_density_type == 1) ? k.init_density : k.init_density / mi;
+    if (S > 1) {
+      const double part = sum;
+      sum = __shfl_sync(gmask, part, gbase);
+#pragma unroll
+      for (int q = 1; q < S; ++q) sum += __shfl_sync(gmask, part, gbase + q);
     }
-    rho[i] = rho_out;
-    if (!(rho_out > 0.0)) atomicOr(err, kErrZeroDensity);
-    if (with_pressure) {
-      const double4_32a vi4 =
-          (si > 0 && k.ncoll > 0) ? colloid_particle_update<D>(k, i, si, x[i], ca) : v[i];
-      write_particle_records<true>(k, i, rho_out, mi, pid[i], vi4, pr, pc, pcf, vf, nn);
+    if (lane_s == 0) {
+      if (kept > cap) atomicOr(err, kErrNeighOverflow);
+      my_max = kept;
+      kept = min(kept, cap);
+      ncount[i] = kept;
+      nhs[i] = min(back, kept);
+      my_pairs = (unsigned long long)kept;
+      const double mi = m[i];
+      double rho_out;
+      if (acc_i) {
+        rho_out = ((k.rhs_density_type == 1) ? k.w0 * mi : k.w0) + sum;
+      } else {
+        rho_out = (k.rhs_density_type == 1) ? k.init_density : k.init_density / mi;
+      }
+      rho[i] = rho_out;
+      if (!(rho_out > 0.0)) atomicOr(err, kErrZeroDensity);
+      if (with_pressure) {
+        const double4_32a vi4 =
+            (si > 0 && k.ncoll > 0) ? colloid_particle_update<D>(k, i, si, x[i], ca) : v[i];
+        write_particle_records<true>(k, i, rho_out, mi, pid[i], vi4, pr, pc, pcf, vf, nn);
+      }
     }
   }
 #pragma unroll
@@ -1200,65 +1170,69 @@ static int grid_for(Handle* h) {
   return g < 1 ? 1 : g;
 }
 
-int verlet_build_gated(Handle* h) {
-  Consts& k = h->k;
+// candidates within sqrt(lim) of every particle into list / count
+static int scan_launch(Handle* h, const int* gate, float lim, uint16_t* list, int* count, int cap,
+                       bool partition) {
   const int g = grid_for(h);
-  if (k.d == 3)
-    k_verlet_build<3><<<g, kWarpsPerBlock * 32, 0, h->stream>>>(
-        k, h->d_rebuild, h->cell_start, h->off, h->vl, h->vcount, h->vcap, h->partitioned ? 1 : 0,
-        h->d_err);
-  else
-    k_verlet_build<2><<<g, kWarpsPerBlock * 32, 0, h->stream>>>(
-        k, h->d_rebuild, h->cell_start, h->off, h->vl, h->vcount, h->vcap, h->partitioned ? 1 : 0,
-        h->d_err);
-  k_rebuild_done<<<1, 1, 0, h->stream>>>(h->d_rebuild);
-  h->launches += 2;
+#define LAUNCH_S(DD)                                                                           \
+  k_scan<DD><<<g, kWarpsPerBlock * 32, 0, h->stream>>>(h->k, gate, h->cell_start, h->off, lim, \
+                                                       list, count, cap, partition ? 1 : 0,    \
+                                                       h->d_err, h->d_stats)
+  if (h->k.d == 3) LAUNCH_S(3); else LAUNCH_S(2);
+#undef LAUNCH_S
+  h->launches++;
   return cuda_check(h, cudaGetLastError(), "candidate list launch") ? MCFG_ECUDA : MCFG_OK;
 }
 
+int verlet_build_gated(Handle* h) {
+  const int rc = scan_launch(h, h->d_rebuild, h->k.rv2f, h->vl, h->vcount, h->vcap, h->partitioned);
+  if (rc) return rc;
+  k_rebuild_done<<<1, 1, 0, h->stream>>>(h->d_rebuild);
+  h->launches++;
+  return cuda_check(h, cudaGetLastError(), "candidate list launch") ? MCFG_ECUDA : MCFG_OK;
+}
+
+// Density of the current particle order.  reuse: over the candidate list of
+// the last rebuild; otherwise the step's own candidates are listed first, in
+// nl, and compacted in place (FP32: within the cut-off by the same test; FP64:
+// with the prefilter's slack, the exact test follows).
 int compute_density(Handle* h, bool with_pressure, bool reuse) {
   Consts& k = h->k;
   cudaStream_t s = h->stream;
+  const int n = (int)h->n;
   if (cuda_check(h, cudaMemsetAsync(h->d_stats, 0, sizeof(int) * 4, s), "memset stats"))
     return MCFG_ECUDA;
   if (cuda_check(h, cudaMemsetAsync(h->d_pairs, 0, sizeof(unsigned long long), s), "memset pairs"))
     return MCFG_ECUDA;
-  const int g = grid_for(h);
+  if (n == 0) return MCFG_OK;
   const bool fp64 = h->p.precision == MCFG_PRECISION_FP64;
-  // FP32 with list reuse: the compact two-segment pair list (sweep32.cu)
-  if (reuse && !fp64) return density_list(h, with_pressure);
-  if (reuse) {
-    const int n = (int)h->n;
-    if (n == 0) return MCFG_OK;
-    const int gr = (n + kReuseTPB - 1) / kReuseTPB;
-#define LAUNCH_R(DD)                                                                            \
-  k_density_reuse<DD><<<gr, kReuseTPB, 0, s>>>(                                                 \
-      k, h->cell_start, h->cell_of, h->x, h->v, h->m, h->sid, h->pid, h->vl, h->vcount, h->nl,  \
+  const uint16_t* vl = reuse ? h->vl : h->nl;
+  const int* vcount = reuse ? h->vcount : h->ncount;
+  if (!reuse) {
+    const int rc = scan_launch(h, nullptr, fp64 ? k.rc2f_hi : k.rc2f, h->nl, h->ncount,
+                               h->neigh_cap, !fp64);
+    if (rc) return rc;
+  }
+  if (!fp64) return density_list(h, with_pressure, vl, vcount, reuse ? h->vcap : h->neigh_cap);
+  const int S = n < kSplit8Below ? 8 : n < kSplitBelow ? 4 : 1;
+  const int gr = (int)(((int64_t)n * S + kReuseTPB - 1) / kReuseTPB);
+#define LAUNCH_R(DD, SS)                                                                        \
+  k_density_reuse<DD, SS><<<gr, kReuseTPB, 0, s>>>(                                             \
+      k, h->cell_start, h->cell_of, h->x, h->v, h->m, h->sid, h->pid, vl, vcount, h->nl,        \
       h->ncount, h->nhs, h->neigh_cap, h->rho, h->pr, h->pc, h->pcf, h->vf,                     \
       with_pressure ? 1 : 0, h->d_err, h->d_stats, h->d_pairs, NN{h->ct, h->act, h->vgt, h->qq}, \
       CollArgs{h->v, h->rxc, h->rxcf})
-    if (k.d == 3)
-      LAUNCH_R(3);
-    else
-      LAUNCH_R(2);
+#define PICK_R(DD)                      \
+  do {                                  \
+    if (S == 8) LAUNCH_R(DD, 8);        \
+    else if (S == 4) LAUNCH_R(DD, 4);   \
+    else LAUNCH_R(DD, 1);               \
+  } while (0)
+  if (k.d == 3) PICK_R(3); else PICK_R(2);
+#undef PICK_R
 #undef LAUNCH_R
-    h->launches++;
-    return cuda_check(h, cudaGetLastError(), "density launch") ? MCFG_ECUDA : MCFG_OK;
-  }
-#define LAUNCH_D(DD, PP)                                                                       \
-  k_density<DD, PP><<<g, kWarpsPerBlock * 32, 0, s>>>(                                          \
-      k, h->cell_start, h->off, h->x, h->v, h->m, h->sid, h->pid, h->nl, h->ncount, h->nhs,    \
-      h->neigh_cap, h->rho, h->pr, h->pc, h->pcf, h->vf, with_pressure ? 1 : 0, h->d_err,      \
-      h->d_stats, h->d_pairs, NN{h->ct, h->act, h->vgt, h->qq}, CollArgs{h->v, h->rxc, h->rxcf})
-  if (k.d == 3) {
-    if (fp64) LAUNCH_D(3, true); else LAUNCH_D(3, false);
-  } else {
-    if (fp64) LAUNCH_D(2, true); else LAUNCH_D(2, false);
-  }
-#undef LAUNCH_D
   h->launches++;
-  if (cuda_check(h, cudaGetLastError(), "density launch")) return MCFG_ECUDA;
-  return MCFG_OK;
+  return cuda_check(h, cudaGetLastError(), "density launch") ? MCFG_ECUDA : MCFG_OK;
 }
 
 int compute_pressure(Handle* h) {

@@ -1,10 +1,11 @@
-// sweep32.cu -- FP32-mixed density sweep over the candidate list.
+// sweep32.cu -- FP32-mixed density sweep over a candidate list.
 //
-// With neighbour-list reuse, a rebuild lists for every particle the
-// candidates within rc + skin (k_verlet_build, pair_kernels.cu), partitioned
-// by species: the fluid partners of a fluid particle first, from row 0 up;
-// every other pair (wall, colloid, or a boundary particle's own pairs) from
-// the last row down.  vcount packs both counts (fluid-fluid | other << 16).
+// The candidates (k_scan, pair_kernels.cu) -- with neighbour-list reuse those
+// within rc + skin at the last rebuild, otherwise the step's own -- are
+// partitioned by species: the fluid partners of a fluid particle first, from
+// row 0 up; every other pair (wall, colloid, or a boundary particle's own
+// pairs) from the last row down.  vcount packs both counts (fluid-fluid |
+// other << 16).  A step's own candidates are compacted in place (vl == nl).
 //
 // Each step the density sweep re-tests every candidate exactly (the FP32
 // test of the per-step scan, same operation order), sums the number
@@ -32,9 +33,8 @@ __global__ void __launch_bounds__(kReuseTPB)
     k_density_list(Consts k, const int* __restrict__ cell_start, const int* __restrict__ cell_of,
                    const float4* __restrict__ off, const double4_32a* __restrict__ x,
                    const double4_32a* __restrict__ v, const double* __restrict__ m,
-                   const int* __restrict__ pid, const uint16_t* __restrict__ vl,
-                   const int* __restrict__ vcount, int vcap, uint16_t* __restrict__ nl,
-                   int* __restrict__ ncount, int cap, double* __restrict__ rho,
+                   const int* __restrict__ pid, const uint16_t* vl, const int* vcount, int vcap,
+                   uint16_t* nl, int* ncount, int cap, double* __restrict__ rho,
                    double* __restrict__ pr, float4* __restrict__ pcf, float4* __restrict__ vf,
                    int with_pressure, unsigned* __restrict__ err, int* __restrict__ stats,
                    unsigned long long* __restrict__ pairs, NN nn, CollArgs ca) {
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(kReuseTPB)
           if (!(t2 < k.rc2f)) continue;
           if (kff + ko < cap) {
             const int row = (p < nff) ? kff : cap - 1 - ko;
-            nl[(size_t)row * n + i] = (uint16_t)entg[u];
+            if (row != cand_row(p, nff, vcap) || nl != vl) nl[(size_t)row * n + i] = (uint16_t)entg[u];
           }
           if (p < nff)
             ++kff;
@@ -213,21 +213,17 @@ __global__ void __launch_bounds__(kReuseTPB)
 
 }  // namespace
 
-int density_list(Handle* h, bool with_pressure) {
+int density_list(Handle* h, bool with_pressure, const uint16_t* vl, const int* vcount, int vcap) {
   Consts& k = h->k;
   cudaStream_t s = h->stream;
   const int n = (int)h->n;
-  if (cuda_check(h, cudaMemsetAsync(h->d_stats, 0, sizeof(int) * 4, s), "memset stats") ||
-      cuda_check(h, cudaMemsetAsync(h->d_pairs, 0, sizeof(unsigned long long), s), "memset pairs"))
-    return MCFG_ECUDA;
-  if (n == 0) return MCFG_OK;
   const bool split = n < kSplitBelow;
   const int S = split ? 4 : 1;
   const int g = (int)(((int64_t)n * S + kReuseTPB - 1) / kReuseTPB);
 #define LAUNCH(DD, SS)                                                                          \
   k_density_list<DD, SS><<<g, kReuseTPB, 0, s>>>(                                              \
-      k, h->cell_start, h->cell_of, h->off, h->x, h->v, h->m, h->pid, h->vl, h->vcount, h->vcap, \
-      h->nl, h->ncount, h->neigh_cap, h->rho, h->pr, h->pcf, h->vf, with_pressure ? 1 : 0,      \
+      k, h->cell_start, h->cell_of, h->off, h->x, h->v, h->m, h->pid, vl, vcount, vcap, h->nl,     \
+      h->ncount, h->neigh_cap, h->rho, h->pr, h->pcf, h->vf, with_pressure ? 1 : 0,             \
       h->d_err, h->d_stats, h->d_pairs, NN{h->ct, h->act, h->vgt, h->qq},                       \
       CollArgs{h->v, h->rxc, h->rxcf})
   if (k.d == 3) {

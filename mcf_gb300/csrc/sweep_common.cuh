@@ -126,6 +126,8 @@ __device__ __forceinline__ void write_particle_records(const Consts& k, int i, d
 constexpr int kReuseTPB = 128;
 // below this many particles the FP32 force sweep runs 4 lanes per particle
 constexpr int64_t kSplitBelow = 50000;
+// and below this many the FP64 density sweep runs 8
+constexpr int64_t kSplit8Below = 12000;
 
 // FP32 offset of each stencil slot (the neighbour cell's origin minus the
 // home cell's, w = Lees-Edwards velocity jump), build_table's t.o, in a

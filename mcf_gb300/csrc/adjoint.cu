@@ -49,7 +49,7 @@ struct Tape {
   int* ncount;
   int* cell_of;      // cell of each particle (ncell: outside the mesh)
   int* cell_start;
-  uint16_t* nl;      // [neigh][n]
+  uint16_t* nl;      // [neigh / 8][n][8]
   double* ct;        // [d*d][n] conformation tensor c' (Oldroyd-B)
   double* vgt;       // [d*d][n] velocity gradient L (Oldroyd-B)
 };
@@ -139,7 +139,7 @@ int alloc_ckpt(Handle* h, AdjBuffers* b, Ckpt& c, bool full) {
 
 int ensure_buffers(Handle* h, int K, int T) {
   const int n = (int)h->n, d = h->k.d, nnw = h->k.newtonian ? 0 : 1;
-  const int ncell = h->k.ncell, neigh = h->neigh_cap;
+  const int ncell = h->k.ncell, neigh = 8 * list_octets(h->neigh_cap, false);
   AdjBuffers* b = h->adj;
   if (b && b->n == n && b->d == d && b->nnw == nnw && b->K == K && b->T == T &&
       b->ncell == ncell && b->neigh == neigh)
@@ -303,7 +303,9 @@ __global__ void k_tape_record(int n, int ncell2, int d2, Tape out, const double4
   out.cell_of[i] = cell_of[i];
   const int c = ncount[i];
   out.ncount[i] = c;
-  for (int e = 0; e < c; ++e) out.nl[(size_t)e * n + i] = nl[(size_t)e * n + i];
+  for (int o = 0; 8 * o < c; ++o)
+    reinterpret_cast<uint4*>(out.nl)[(size_t)o * n + i] =
+        reinterpret_cast<const uint4*>(nl)[(size_t)o * n + i];
   if (out.ct)
     for (int q = 0; q < d2; ++q) {
       out.ct[(size_t)q * n + i] = ct[(size_t)q * n + i];
@@ -468,7 +470,7 @@ __global__ void __launch_bounds__(kAdjTPB)
   double Bbar = 0.0, Abar = 0.0, nbL = 0.0, etab = 0.0;
   const int cnt = live ? tp.ncount[il] : 0;
   for (int e = part; e < cnt; e += split) {
-    const int ent = tp.nl[(size_t)e * n + il];
+    const int ent = tp.nl[up_at(e, n, il)];
     const int sl = ent >> kLocalBits, q = ent & (kMaxCellCount - 1);
     const int j = s_start[sl * kAdjTPB + tid] + q;
     const double4_32a xj4 = tp.x[j];
@@ -680,7 +682,7 @@ __global__ void __launch_bounds__(kAdjTPB)
   double acc[3] = {0, 0, 0};
   const int cnt = live ? tp.ncount[i] : 0;
   for (int e = part; e < cnt; e += split) {
-    const int ent = tp.nl[(size_t)e * n + i];
+    const int ent = tp.nl[up_at(e, n, i)];
     const int sl = ent >> kLocalBits, q = ent & (kMaxCellCount - 1);
     const int j = s_start[sl * kAdjTPB + tid] + q;
     const double4_32a xj4 = tp.x[j];

@@ -9,6 +9,7 @@
 #include <string>
 
 #include "mcfg_internal.cuh"
+#include "pair_common.cuh"
 #include "sph.cuh"
 
 using namespace mcfg;
@@ -154,7 +155,7 @@ void free_all(Handle* h) {
   void* ptrs[] = {h->x, h->v, h->f, h->m, h->pid, h->sid, h->hidx, h->rho, h->pr, h->st,
                   h->x2, h->v2, h->f2, h->m2, h->pid2, h->sid2, h->hidx2, h->key, h->rank,
                   h->cnt, h->cell_start, h->scan_part, h->order, h->off, h->cell_of, h->nl,
-                  h->ncount, h->nhs, h->jp, h->pc, h->pcf, h->vf, h->wd, h->red, h->d_err, h->d_stats, h->d_pairs,
+                  h->ncount, h->nhs, h->jp, h->pc, h->vf, h->wd, h->red, h->d_err, h->d_stats, h->d_pairs,
                   h->up_x, h->up_v, h->up_m, h->up_id, h->ct, h->act, h->vgt, h->ct2,
                   h->act2, h->qq, h->coll, h->coll_start, h->coll_mem, h->slot_of, h->rxc,
                   h->rxcf, h->coll_out, h->crec, h->cxnew};
@@ -331,6 +332,10 @@ void make_consts(const mcfg_params& p, Consts& k) {
   k.gamma = p.gamma;
   if (p.stateEquation_type == 2)  // stateEquation_new.F90:102-103
     k.p0 = p.c * p.c * p.rho * std::pow(p.rho_ref / p.rho, p.gamma) / p.gamma;
+  k.c2f = (float)k.c2;
+  k.rho_reff = (float)k.rho_ref;
+  k.gammaf = (float)k.gamma;
+  k.p0f = (float)k.p0;
   k.eta = p.eta;
   k.eta_coef = p.eta_coef;
   k.kt = p.kt;
@@ -506,6 +511,7 @@ int ensure_capacity(Handle* h, int64_t n64) {
       neigh = std::min((neigh + 7) / 8 * 8, 4096);
     }
     h->neigh_cap = neigh;
+    const bool two = h->p.precision != MCFG_PRECISION_FP64;  // list segments
     const int nbins = h->k.ncell + 1;
     const int ntiles = (nbins + 4095) / 4096 + 1;
     if ((rc = dalloc(h, &h->x, cap)) || (rc = dalloc(h, &h->v, cap)) ||
@@ -520,7 +526,7 @@ int ensure_capacity(Handle* h, int64_t n64) {
         (rc = dalloc(h, &h->order, cap)) || (rc = dalloc(h, &h->off, cap)) ||
         (rc = dalloc(h, &h->cell_of, cap)) || (rc = dalloc(h, &h->ncount, cap)) ||
         (rc = dalloc(h, &h->nhs, cap)) || (rc = dalloc(h, &h->slot_of, cap)) ||
-        (rc = dalloc(h, &h->nl, cap * (size_t)neigh)) ||
+        (rc = dalloc(h, &h->nl, cap * (size_t)(8 * list_octets(neigh, two)))) ||
         (rc = dalloc(h, &h->cnt, (size_t)nbins + 1)) ||
         (rc = dalloc(h, &h->cell_start, (size_t)nbins + 2)) ||
         (rc = dalloc(h, &h->scan_part, (size_t)ntiles + 1)) ||
@@ -532,7 +538,8 @@ int ensure_capacity(Handle* h, int64_t n64) {
       // candidates within rc + skin: the list grows with the volume ratio
       const double rv = std::sqrt((double)h->k.rv2f) / h->p.cut_off;
       h->vcap = (int)std::ceil(neigh * std::pow(rv, d) * 1.05) + 8;
-      if ((rc = dalloc(h, &h->x_ref, cap)) || (rc = dalloc(h, &h->vl, cap * (size_t)h->vcap)) ||
+      if ((rc = dalloc(h, &h->x_ref, cap)) ||
+          (rc = dalloc(h, &h->vl, cap * (size_t)(8 * list_octets(h->vcap, two)))) ||
           (rc = dalloc(h, &h->vcount, cap)) || (rc = dalloc(h, &h->d_rebuild, 2)))
         return rc;
       h->partitioned = h->p.precision != MCFG_PRECISION_FP64;
@@ -544,9 +551,8 @@ int ensure_capacity(Handle* h, int64_t n64) {
       if ((rc = dalloc(h, &h->pc, cap)) || (rc = dalloc(h, &h->rxc, cap))) return rc;
     } else {
       if ((rc = dalloc(h, &h->rxcf, cap))) return rc;
-      if ((rc = dalloc(h, &h->pcf, cap)) || (rc = dalloc(h, &h->vf, cap)) ||
-          (rc = dalloc(h, &h->wd, cap)))
-        return rc;
+      if ((rc = dalloc(h, &h->vf, 2 * cap)) || (rc = dalloc(h, &h->wd, cap))) return rc;
+      h->pcf = h->vf + 1;
     }
     if (!h->p.Newtonian) {
       const size_t d2 = (size_t)d * d;

@@ -63,6 +63,7 @@ struct Consts {
   // FP32 copies of the pair constants (the FP32 path never converts from
   // double inside a pair loop: GB300's FP64 pipe is narrow)
   float etaf, eta_coeff, ktf;
+  float c2f, rho_reff, gammaf, p0f;  // equation of state
   float wall_vf[6][3];   // FP32 copy of wall_v
   int wall_axis;         // the single solid-wall axis, -1 if none, -2 if several
   // moving boundaries (boundary_update_boundary.F90): wall_v holds MCF's
@@ -203,16 +204,17 @@ struct Handle {
   float4* off = nullptr;     // FP32 offset to the cell origin, w = cell id
   int* cell_of = nullptr;    // cell per sorted particle (ncell = outside)
   // ---- neighbours ----
-  uint16_t* nl = nullptr;    // [neigh_cap][cap] entries slot<<11|local; FP32 list reuse:
-                             // fluid-fluid pairs from row 0 up, the others from the
-                             // last row down, ncount = fluid-fluid | other << 16
+  uint16_t* nl = nullptr;    // the step's pairs, entries slot<<11|local in octets
+                             // [list_octets(neigh_cap)][n][8] (pair_common.cuh); FP32:
+                             // two segments, ncount = fluid-fluid | other << 16
   int* ncount = nullptr;     // [cap]
   int* nhs = nullptr;        // [cap] first entry of the owned (forward) half
   void* jp = nullptr;        // symmetric force partial sums [(NSF+1)*3][cap] (T)
   // ---- pair records ----
   double4_32a* pc = nullptr;     // FP64 path: (p/n^2 or p, 1/n^2, 1/m, rho)
-  float4* pcf = nullptr;     // FP32 path: same in float
-  float4* vf = nullptr;      // FP32 path: velocity (w = packed id bits)
+  float4* vf = nullptr;      // FP32 path: [2 i] velocity (w = packed id bits) and
+                             // [2 i + 1] the pair coefficients in float
+  float4* pcf = nullptr;     // vf + 1
   float2* wd = nullptr;      // FP32 path: signed distances to the wall-axis faces
   // ---- reductions & errors ----
   double* red = nullptr;     // block partials
@@ -228,10 +230,8 @@ struct Handle {
   size_t up_cap = 0;
   // ---- neighbour-list reuse ----
   double4_32a* x_ref = nullptr;  // positions at the last rebuild
-  uint16_t* vl = nullptr;        // [vcap][n] candidates within rc + skin (slot<<11 | local);
-                                 // FP32 handles: fluid-fluid pairs from row 0 up, the
-                                 // others from row vcap-1 down (sweep32.cu)
-  bool partitioned = false;      // FP32 lists: fluid-fluid rows up, the others down
+  uint16_t* vl = nullptr;        // candidates within rc + skin, laid out as nl
+  bool partitioned = false;      // FP32 lists: fluid-fluid candidates, then the others
   int* vcount = nullptr;         // [n]
   int vcap = 0;
   int* d_rebuild = nullptr;      // [0] rebuild request, [1] rebuilds done
@@ -354,6 +354,10 @@ int compute_pressure(Handle* h);
 int compute_force(Handle* h, int64_t step, int fuse_mode, double dt);
 // FP32-mixed density over a partitioned candidate list (sweep32.cu)
 int density_list(Handle* h, bool with_pressure, const uint16_t* vl, const int* vcount, int vcap);
+// FP32-mixed force of the common forms, two pairs an instruction (force32.cu);
+// false: another sweep has to run
+bool force32_packed(Handle* h, uint32_t step, const int64_t* step_ptr, float inv_sqdt,
+                    int fuse_mode, double dt);
 int apply_body_force(Handle* h);
 int integrate_velocity(Handle* h, double dt, double lambda);
 int integrate_position(Handle* h, double dt);

@@ -7,6 +7,59 @@ namespace mcfg {
 
 constexpr int kWarpsPerBlock = 4;
 
+// Neighbour and candidate lists: octets of entries, [octet][particle][8], so
+// that a thread takes eight of its entries with one 16-byte load (coalesced
+// across lanes) well before it needs them; with one 2-byte load an entry the
+// FP32 sweeps spent half of their time waiting for the list.  Entry r of the
+// first segment lies in octet r / 8 from the first one up, of the second
+// segment (FP32 lists: pairs with a boundary particle) from the last one down.
+// With two segments there are two octets more than cap / 8: both may end in a
+// partial one.
+__host__ __device__ constexpr int list_octets(int cap, bool two = true) {
+  return two ? cap / 8 + 2 : (cap + 7) / 8;
+}
+__device__ __forceinline__ size_t up_at(int r, int n, int i) {
+  return ((unsigned long long)((unsigned)r >> 3) * (unsigned)n + i) * 8 + (r & 7);
+}
+__device__ __forceinline__ size_t down_at(int r, int cap, int n, int i) {
+  return ((unsigned long long)(unsigned)(list_octets(cap) - 1 - (r >> 3)) * (unsigned)n + i) * 8 +
+         (r & 7);
+}
+// logical entry e of a list whose first segment holds nff
+__device__ __forceinline__ size_t entry_at(int e, int nff, int cap, int n, int i) {
+  return e < nff ? up_at(e, n, i) : down_at(e - nff, cap, n, i);
+}
+
+// A thread's appends to one segment, four entries a store.
+struct ListTail {
+  unsigned lo = 0, hi = 0;  // the last four entries, the newest on top
+  int count = 0;
+  __device__ __forceinline__ void push(unsigned ent) {
+    lo = __byte_perm(lo, hi, 0x5432);
+    hi = __byte_perm(hi, ent, 0x5432);
+    ++count;
+  }
+  // entries 4 q .. 4 q + 3 of the segment (up: from the first octet)
+  __device__ __forceinline__ static void put(uint16_t* list, bool up, int q, int octets, int n,
+                                             int i, uint2 w) {
+    const int o = q >> 1;
+    if (o >= octets) return;  // past the capacity: the overflow is an error already
+    const unsigned row = (unsigned)(up ? o : octets - 1 - o);
+    reinterpret_cast<uint2*>(list)[((unsigned long long)row * (unsigned)n + i) * 2 + (q & 1)] = w;
+  }
+  __device__ __forceinline__ bool full() const { return (count & 3) == 0; }
+  __device__ __forceinline__ void store(uint16_t* list, bool up, int octets, int n, int i) const {
+    put(list, up, (count >> 2) - 1, octets, n, i, make_uint2(lo, hi));
+  }
+  // the last, partial group
+  __device__ __forceinline__ void finish(uint16_t* list, bool up, int octets, int n, int i) const {
+    const int r = count & 3;
+    if (r == 0) return;
+    const unsigned long long w = (((unsigned long long)hi << 32) | lo) >> (16 * (4 - r));
+    put(list, up, count >> 2, octets, n, i, make_uint2((unsigned)w, (unsigned)(w >> 32)));
+  }
+};
+
 struct NbTable {
   int start[kMaxStencil];
   int count[kMaxStencil];
@@ -281,6 +334,37 @@ __device__ __forceinline__ void build_lane_table(const Consts& k, int cell,
     s_start[s * TPB + t] = (nc >= 0) ? cell_start[nc] : 0;
     if (SHIFT) s_shift[s * TPB + t] = sh;
   }
+}
+
+// The same table for S adjacent lanes that share a particle: TPB / S columns,
+// the lanes of a group build every S-th slot of theirs (group mask gmask).
+template <int D, int TPB, int S>
+__device__ __forceinline__ void build_group_table(const Consts& k, int cell,
+                                                  const int* __restrict__ cell_start,
+                                                  int* __restrict__ s_start, unsigned gmask) {
+  constexpr int CENTER = (D == 3) ? 13 : 4;
+  const int g = threadIdx.x / S;
+  int c[3] = {0, 0, 0};
+  if (cell < k.ncell) cell_coords<D>(k, cell, c);
+  const int st = le_state(k, c[1]);
+  for (int s = threadIdx.x % S; s < k.ns; s += S) {
+    int start = 0;
+    if (cell == k.ncell) {
+      if (s == CENTER) start = cell_start[cell];
+    } else {
+      int sh;
+      const int nc = slot_cell<D>(k, c, s, st, sh);
+      if (nc >= 0) start = cell_start[nc];
+    }
+    s_start[s * (TPB / S) + g] = start;
+  }
+  __syncwarp(gmask);
+}
+
+// the lanes of a thread's group of S
+template <int S>
+__device__ __forceinline__ unsigned group_mask() {
+  return (S == 32 ? 0xffffffffu : (1u << S) - 1u) << ((threadIdx.x & 31) & ~(S - 1));
 }
 
 }  // namespace mcfg

@@ -4,9 +4,8 @@
 //
 // Candidates (k_scan): one warp owns one cell and walks its particles in
 // chunks of 32 (lane = particle i) through the 27 (3D) or 9 (2D) neighbour
-// cells, an FP32 test on cell offsets; the hits go to a per-particle list
-// [capacity][N] of 16-bit entries slot<<11 | local index (coalesced across
-// lanes).  With list reuse the list holds the candidates within rc + skin and
+// cells, an FP32 test on cell offsets; the hits go to a per-particle list of
+// 16-bit entries slot<<11 | local index (octets, see pair_common.cuh).  With list reuse the list holds the candidates within rc + skin and
 // outlives the step, otherwise it is made for this step.
 //
 // Density (k_density_reuse here for FP64, k_density_list in sweep32.cu for
@@ -39,9 +38,11 @@ namespace mcfg {
 constexpr int kMaskRows = 32;  // candidate chunks a warp notes between two emissions
 
 // Candidates of every particle with FP32 squared distance below lim, in slot
-// order and particle order, into list ([cap][n] rows) and count.  With
-// partition (FP32 lists) the fluid-fluid candidates fill the rows from 0 up,
-// the others from the last row down, and count = fluid-fluid | other << 16.
+// order and particle order, into list and count.  With partition (FP32 lists)
+// the fluid-fluid candidates form the first segment, the others the second,
+// and count = fluid-fluid | other << 16.  EXACT: the separation is formed as
+// the density sweep forms it, so that lim decides alike (a step's own FP32
+// list); the other lists have slack in lim and save that addition.
 // gate: return at once when *gate is zero (no rebuild due).
 //
 // Bound: instruction issue (a 3D particle meets 27 cells of ~28 particles, of
@@ -49,12 +50,11 @@ constexpr int kMaskRows = 32;  // candidate chunks a warp notes between two emis
 // memory as separate coordinates, tested two at a time by packed FP32
 // arithmetic against broadcast loads, and leaves one hit bit a candidate (the
 // sign of d2 - lim, shifted in): ~6 instructions a test with nothing done a
-// hit.  The bits are expanded afterwards, lanes near the same list row, so the
-// 2-byte stores coalesce (expanding chunk by chunk takes fewer instructions
-// but scatters them: 270 us).  The next chunk is in flight meanwhile.
-// 261,568 particles: 196 us (tests 113, expansion 83) where writing each hit
-// as it was found took 344 us.
-template <int D>
+// hit.  The bits are expanded afterwards, four entries a store.  The next
+// chunk is in flight meanwhile.  261,568
+// particles: 196 us (tests 113, expansion 83) where writing each hit as it was
+// found took 344 us.
+template <int D, bool EXACT>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     k_scan(Consts k, const int* __restrict__ gate, const int* __restrict__ cell_start,
            const float4* __restrict__ off, float lim, uint16_t* __restrict__ list,
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   __shared__ unsigned s_fluid[kWarpsPerBlock][kMaskRows];
   __shared__ int s_ent[kWarpsPerBlock][kMaskRows];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = k.n, ns = k.ns;
+  const int n = k.n, ns = k.ns, octets = list_octets(cap, partition != 0);
   const F2 neg_lim = splat2(-lim);
   for (int cell = blockIdx.x * kWarpsPerBlock + wib; cell <= k.ncell;
        cell += gridDim.x * kWarpsPerBlock) {
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
       const bool active = i < c1;
       const float4 oi = active ? off[i] : make_float4(0.f, 0.f, 0.f, 0.f);
       const bool fluid_i = __float_as_int(oi.w) == 0;
-      int cnt = 0, cnt_o = 0;  // cnt_o: partitioned lists' second segment
+      ListTail ff, other;  // the two segments
       int rows = 0, buf = 0;
       // one segment only: no partition, or all particles met are fluid
       const bool plain0 = !partition || __all_sync(0xffffffffu, fluid_i);
@@ -111,18 +111,30 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
         __syncwarp();
         nx = (sl < ns && b2 + lane < jn) ? off[t.start[sl] + b2 + lane] : pad;
         const float4 so = t.o[sl_c];
-        const F2 px = splat2(oi.x - so.x), py = splat2(oi.y - so.y), pz = splat2(oi.z - so.z);
+        const F2 px = splat2(EXACT ? oi.x : oi.x - so.x), py = splat2(EXACT ? oi.y : oi.y - so.y),
+                 pz = splat2(EXACT ? oi.z : oi.z - so.z);
+        const F2 sx = splat2(-so.x), sy = splat2(-so.y), sz = splat2(-so.z);
         unsigned mask = 0;
         int q = 0;
         for (; q < mm; q += 4) {
           const ulonglong2 x4 = *reinterpret_cast<const ulonglong2*>(&sc[0][q]);
           const ulonglong2 y4 = *reinterpret_cast<const ulonglong2*>(&sc[1][q]);
-          const F2 xa = add2(px, F2{x4.x}), xb = add2(px, F2{x4.y});
-          const F2 ya = add2(py, F2{y4.x}), yb = add2(py, F2{y4.y});
+          F2 xa = add2(px, F2{x4.x}), xb = add2(px, F2{x4.y});
+          F2 ya = add2(py, F2{y4.x}), yb = add2(py, F2{y4.y});
+          if (EXACT) {
+            xa = add2(xa, sx);
+            xb = add2(xb, sx);
+            ya = add2(ya, sy);
+            yb = add2(yb, sy);
+          }
           F2 da = fma2(ya, ya, mul2(xa, xa)), db = fma2(yb, yb, mul2(xb, xb));
           if (D == 3) {
             const ulonglong2 z4 = *reinterpret_cast<const ulonglong2*>(&sc[2][q]);
-            const F2 za = add2(pz, F2{z4.x}), zb = add2(pz, F2{z4.y});
+            F2 za = add2(pz, F2{z4.x}), zb = add2(pz, F2{z4.y});
+            if (EXACT) {
+              za = add2(za, sz);
+              zb = add2(zb, sz);
+            }
             da = fma2(za, za, da);
             db = fma2(zb, zb, db);
           }
@@ -154,11 +166,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
         if (rows == kMaskRows || sl >= ns) {
           // expand the bits, each lane its own rows in order
           __syncwarp();
-          int r = -1, ent0 = 0, left = cap - cnt - cnt_o;
+          int r = -1, ent0 = 0;
           unsigned m = 0;
           if (plain) {
-            const int before = left;
-            uint16_t* dst = list + (size_t)cnt * n + i;
             for (;;) {
               while (m == 0 && r + 1 < rows) {
                 ++r;
@@ -168,23 +178,23 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
               if (m == 0) break;
               const int c = __clz(m);
               m ^= 0x80000000u >> c;
-              if (left > 0) *dst = (uint16_t)(ent0 + c);
-              dst += n;
-              --left;
+              ff.push(ent0 + c);
+              if (ff.full()) ff.store(list, true, octets, n, i);
             }
-            cnt += before - left;
           } else {
             for (;;) {
               while (m == 0 && r + 1 < rows) m = s_mask[wib][++r][lane];
               if (m == 0) break;
               const int c = __clz(m);
               m ^= 0x80000000u >> c;
-              const bool ff = fluid_i && ((s_fluid[wib][r] << c) >> 31);
-              if (left > 0)
-                list[(size_t)(ff ? cnt : cap - 1 - cnt_o) * n + i] = (uint16_t)(s_ent[wib][r] + c);
-              cnt += ff ? 1 : 0;
-              cnt_o += ff ? 0 : 1;
-              --left;
+              const unsigned ent = s_ent[wib][r] + c;
+              if (fluid_i && ((s_fluid[wib][r] << c) >> 31)) {
+                ff.push(ent);
+                if (ff.full()) ff.store(list, true, octets, n, i);
+              } else {
+                other.push(ent);
+                if (other.full()) other.store(list, false, octets, n, i);
+              }
             }
           }
           plain = plain0;
@@ -193,7 +203,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
         }
       }
       if (active) {
+        ff.finish(list, true, octets, n, i);
+        other.finish(list, false, octets, n, i);
+        int cnt = ff.count, cnt_o = other.count;
         if (cnt + cnt_o > cap) {
+          // the counts are cut to what fits (every entry below them holds a
+          // candidate of this particle), the overflow is reported
           atomicOr(err, kErrNeighOverflow);
           atomicMax(&stats[1], cnt + cnt_o);
           cnt = min(cnt, cap);
@@ -261,7 +276,7 @@ __global__ void __launch_bounds__(kReuseTPB)
       bool in = false, fwd = false;
       int ent = 0;
       if (S == 1 || e < cnt) {
-        ent = vl[(size_t)e * n + i];
+        ent = vl[up_at(e, n, i)];
         const int sl = ent >> kLocalBits, q = ent & (kMaxCellCount - 1);
         const int j = s_start[sl * kReuseTPB + tid] + q;
         const double4_32a xj4 = x[j];
@@ -277,7 +292,7 @@ __global__ void __launch_bounds__(kReuseTPB)
       }
       if (S == 1) {
         if (!in) continue;
-        if (kept < cap) nl[(size_t)kept * n + i] = (uint16_t)ent;
+        if (kept < cap) nl[up_at(kept, n, i)] = (uint16_t)ent;
         ++kept;
         back += fwd ? 0 : 1;
       } else {
@@ -285,7 +300,7 @@ __global__ void __launch_bounds__(kReuseTPB)
         const unsigned bi = (__ballot_sync(gmask, in) & gmask) >> gbase;
         const unsigned bf = (__ballot_sync(gmask, in && !fwd) & gmask) >> gbase;
         const int pos = kept + __popc(bi & ((1u << lane_s) - 1u));
-        if (in && pos < cap) nl[(size_t)pos * n + i] = (uint16_t)ent;
+        if (in && pos < cap) nl[up_at(pos, n, i)] = (uint16_t)ent;
         kept += __popc(bi);
         back += __popc(bf);
       }
@@ -392,7 +407,7 @@ __global__ void __launch_bounds__(kReuseTPB)
   for (int a = 0; a < 9; ++a) sacc[a] = 0;
   const int cnt = ncount[i];
   for (int e = 0; e < cnt; ++e) {
-    const int ent = nl[(size_t)e * n + i];
+    const int ent = nl[up_at(e, n, i)];
     const int sl = ent >> kLocalBits, q = ent & (kMaxCellCount - 1);
     const int j = s_start[sl * kReuseTPB + threadIdx.x] + q;
     const int sj = sid[j];
@@ -549,25 +564,6 @@ __global__ void __launch_bounds__(kReuseTPB)
 // FP32-mixed force sweep: pair arithmetic in FP32 on cell offsets, Kahan
 // sums, the next pair's data loaded while the current one is computed.
 // ---------------------------------------------------------------------------
-struct JData {
-  float4 o, v, c;
-  int sl, j;
-};
-
-template <int D>
-__device__ __forceinline__ JData load_j(const int* __restrict__ s_start, int ent,
-                                        const float4* __restrict__ off,
-                                        const float4* __restrict__ vf,
-                                        const float4* __restrict__ pcf) {
-  JData d;
-  d.sl = ent >> kLocalBits;
-  d.j = s_start[d.sl * kReuseTPB + threadIdx.x] + (ent & (kMaxCellCount - 1));
-  d.o = off[d.j];
-  d.v = vf[d.j];
-  d.c = pcf[d.j];
-  return d;
-}
-
 // S lanes per particle (1, or 4 for small systems, where one thread per
 // particle leaves most of the GPU idle and each thread's serial pair loop
 // sets the time): lane l takes list entries l, l + S, ...; the lanes' sums
@@ -582,7 +578,7 @@ __global__ void __launch_bounds__(kReuseTPB, (NNW && D == 3) ? 4 : 5)
               const uint16_t* __restrict__ nl, const int* __restrict__ ncount, int cap,
               const float4* __restrict__ off,
               const double4_32a* __restrict__ x, const double4_32a* __restrict__ v,
-              const float4* __restrict__ pcf, const float4* __restrict__ vf,
+              const float4* __restrict__ vf,
               const float2* __restrict__ wd, double4_32a* __restrict__ f,
               double* __restrict__ st, int fuse_mode, double dt,
               double4_32a* __restrict__ v_out, uint32_t step_arg,
@@ -608,9 +604,9 @@ __global__ void __launch_bounds__(kReuseTPB, (NNW && D == 3) ? 4 : 5)
   const float4* slot_tab = slot_table(k, s_slot, celli);
   const float4 oi = off[i];
   const int si = __float_as_int(oi.w);
-  const float4 v4i = vf[i];
+  float4 v4i, ci;
+  load_vc(vf, i, v4i, ci);
   const int pidi = __float_as_int(v4i.w);
-  const float4 ci = pcf[i];
   const float2 wdi = (walls && k.wall_axis >= 0) ? wd[i] : make_float2(0.f, 0.f);
   constexpr bool nnw = NNW;  // Oldroyd-B terms compiled only when used
   const float* qq = (const float*)nn.qq;
@@ -625,20 +621,19 @@ __global__ void __launch_bounds__(kReuseTPB, (NNW && D == 3) ? 4 : 5)
   T sacc[9];
 #pragma unroll
   for (int a = 0; a < 9; ++a) sacc[a] = 0.f;
-  // the list's two segments (fluid-fluid pairs from row 0 up, the others
-  // from row cap-1 down; a per-step list has only the first)
+  // the list's two segments: fluid-fluid pairs, then the others
   const int nc = ncount[i];
   const int nff = nc & 0xffff, cnt = nff + (nc >> 16);
   JData nxt;
   int ent_n1 = 0;
   if (lane_s < cnt)
-    nxt = load_j<D>(s_start, nl[(size_t)cand_row(lane_s, nff, cap) * n + i], off, vf, pcf);
-  if (lane_s + S < cnt) ent_n1 = nl[(size_t)cand_row(lane_s + S, nff, cap) * n + i];
+    nxt = load_j(s_start, nl[entry_at(lane_s, nff, cap, n, i)], off, vf);
+  if (lane_s + S < cnt) ent_n1 = nl[entry_at(lane_s + S, nff, cap, n, i)];
   for (int e = lane_s; e < cnt; e += S) {
     const JData cur = nxt;
     if (e + S < cnt) {
-      nxt = load_j<D>(s_start, ent_n1, off, vf, pcf);
-      if (e + 2 * S < cnt) ent_n1 = nl[(size_t)cand_row(e + 2 * S, nff, cap) * n + i];
+      nxt = load_j(s_start, ent_n1, off, vf);
+      if (e + 2 * S < cnt) ent_n1 = nl[entry_at(e + 2 * S, nff, cap, n, i)];
     }
     const int sj = __float_as_int(cur.o.w);
     if (si != 0 && sj != 0 && !(si > 0 && sj > 0 && si != sj && k.pp_cc)) continue;
@@ -663,97 +658,9 @@ __global__ void __launch_bounds__(kReuseTPB, (NNW && D == 3) ? 4 : 5)
         qie[cc] = qi[cc];
       }
     }
-    if (si < 0 || sj < 0) {
-      // fluid-wall pair: the wall particle takes the Morris no-slip
-      // velocity and the fluid pressure (pp_interaction_fw.inc / _wf.inc),
-      // in the Oldroyd-B model also the fluid density and pressure
-      // tensor; face distances come from the FP64-rounded per-particle
-      // values (one wall axis) or from the FP64 positions (several)
-      const int sw = (sj < 0) ? sj : si;
-      const int face = -sw;
-      const bool lower = (face & 1) != 0;
-      float df, dw;
-      if (k.wall_axis >= 0) {
-        const float2 wj = wd[cur.j];
-        const float di = lower ? wdi.x : wdi.y, dj = lower ? wj.x : wj.y;
-        df = (sj < 0) ? di : dj;
-        dw = (sj < 0) ? dj : di;
-      } else {
-        const int axis = (face - 1) >> 1;
-        const double x_sur = axis == 0 ? (lower ? k.min_phys[0] : k.max_phys[0])
-                             : axis == 1 ? (lower ? k.min_phys[1] : k.max_phys[1])
-                                         : (lower ? k.min_phys[2] : k.max_phys[2]);
-        const double4_32a a4 = x[i], b4 = x[cur.j];
-        const double xa = axis == 0 ? a4.x : axis == 1 ? a4.y : a4.z;
-        const double xb = axis == 0 ? b4.x : axis == 1 ? b4.y : b4.z;
-        df = (float)(((sj < 0) ? xa : xb) - x_sur);
-        dw = (float)(((sj < 0) ? xb : xa) - x_sur);
-      }
-      T vw[3];
-      if (sj < 0) {
-        wall_noslip_dist<T, D>(k, df, dw, vi, sj, vw);
-#pragma unroll
-        for (int a = 0; a < D; ++a) vj[a] = vw[a];
-        if (nnw) {
-          Aj = Ai;
-          Bj = Bi;
-#pragma unroll
-          for (int cc = 0; cc <= D2; ++cc) qj[cc] = qi[cc];
-        } else {
-          Aj = boundary_A<T>(k.rhs_force_type, ci.w, cur.c.y);
-        }
-      } else {
-        wall_noslip_dist<T, D>(k, df, dw, vj, si, vw);
-#pragma unroll
-        for (int a = 0; a < D; ++a) vi[a] = vw[a];
-        if (nnw) {
-          Ai = Aj;
-          Bi = Bj;
-#pragma unroll
-          for (int cc = 0; cc <= D2; ++cc) qie[cc] = qj[cc];
-        } else {
-          Ai = boundary_A<T>(k.rhs_force_type, cur.c.w, ci.y);
-        }
-      }
-    } else if ((si > 0) != (sj > 0)) {
-      // fluid-colloid pair (pp_interaction_fc.inc / _cf.inc)
-      if (sj > 0) {
-        if (k.coll_noslip == 2) {
-          const float4 rc4 = ca.rxcf[cur.j];
-          const T rxc_[3] = {rc4.x, rc4.y, rc4.z};
-          T vw[3];
-          colloid_noslip<T, D>(k, sj - 1, rxc_, r, vi, vw);
-#pragma unroll
-          for (int a = 0; a < D; ++a) vj[a] = vw[a];
-        }
-        if (nnw) {
-          Aj = Ai;
-          Bj = Bi;
-#pragma unroll
-          for (int cc = 0; cc <= D2; ++cc) qj[cc] = qi[cc];
-        } else {
-          Aj = boundary_A<T>(k.rhs_force_type, ci.w, cur.c.y);
-        }
-      } else {
-        if (k.coll_noslip == 2) {
-          const float4 rc4 = ca.rxcf[i];
-          const T rxc_[3] = {rc4.x, rc4.y, rc4.z};
-          const T rfc[3] = {-r[0], -r[1], -r[2]};
-          T vw[3];
-          colloid_noslip<T, D>(k, si - 1, rxc_, rfc, vj, vw);
-#pragma unroll
-          for (int a = 0; a < D; ++a) vi[a] = vw[a];
-        }
-        if (nnw) {
-          Ai = Aj;
-          Bi = Bj;
-#pragma unroll
-          for (int cc = 0; cc <= D2; ++cc) qie[cc] = qj[cc];
-        } else {
-          Ai = boundary_A<T>(k.rhs_force_type, cur.c.w, ci.y);
-        }
-      }
-    }
+    if (si < 0 || sj < 0 || (si > 0) != (sj > 0))
+      boundary_pair32<D, NNW>(k, i, cur.j, si, sj, r, wdi, wd, x, ca, ci.w, cur.c.w, vi, vj, Ai,
+                              Aj, Bi, Bj, qi, qie, qj);
     const T gw = kernel_gradw<T>(k, d);
     T vij[3];
 #pragma unroll
@@ -981,7 +888,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
           if (valid) {
             const int ii = base + ow_l;
             const int e = e0s[ow_l] + (fidx - ex[ow_l]);
-            const int ent = nl[(size_t)e * n + ii];
+            const int ent = nl[up_at(e, n, ii)];
             jsl = ent >> kLocalBits;
             jq = ent & (kMaxCellCount - 1);
             const int j = t.start[jsl] + jq;
@@ -1172,20 +1079,25 @@ static int grid_for(Handle* h) {
 
 // candidates within sqrt(lim) of every particle into list / count
 static int scan_launch(Handle* h, const int* gate, float lim, uint16_t* list, int* count, int cap,
-                       bool partition) {
+                       bool partition, bool exact) {
   const int g = grid_for(h);
-#define LAUNCH_S(DD)                                                                           \
-  k_scan<DD><<<g, kWarpsPerBlock * 32, 0, h->stream>>>(h->k, gate, h->cell_start, h->off, lim, \
-                                                       list, count, cap, partition ? 1 : 0,    \
-                                                       h->d_err, h->d_stats)
-  if (h->k.d == 3) LAUNCH_S(3); else LAUNCH_S(2);
+#define LAUNCH_S(DD, EX)                                                                          \
+  k_scan<DD, EX><<<g, kWarpsPerBlock * 32, 0, h->stream>>>(h->k, gate, h->cell_start, h->off, lim, \
+                                                           list, count, cap, partition ? 1 : 0,    \
+                                                           h->d_err, h->d_stats)
+  if (h->k.d == 3) {
+    if (exact) LAUNCH_S(3, true); else LAUNCH_S(3, false);
+  } else {
+    if (exact) LAUNCH_S(2, true); else LAUNCH_S(2, false);
+  }
 #undef LAUNCH_S
   h->launches++;
   return cuda_check(h, cudaGetLastError(), "candidate list launch") ? MCFG_ECUDA : MCFG_OK;
 }
 
 int verlet_build_gated(Handle* h) {
-  const int rc = scan_launch(h, h->d_rebuild, h->k.rv2f, h->vl, h->vcount, h->vcap, h->partitioned);
+  const int rc = scan_launch(h, h->d_rebuild, h->k.rv2f, h->vl, h->vcount, h->vcap, h->partitioned,
+                             false);
   if (rc) return rc;
   k_rebuild_done<<<1, 1, 0, h->stream>>>(h->d_rebuild);
   h->launches++;
@@ -1210,7 +1122,7 @@ int compute_density(Handle* h, bool with_pressure, bool reuse) {
   const int* vcount = reuse ? h->vcount : h->ncount;
   if (!reuse) {
     const int rc = scan_launch(h, nullptr, fp64 ? k.rc2f_hi : k.rc2f, h->nl, h->ncount,
-                               h->neigh_cap, !fp64);
+                               h->neigh_cap, !fp64, !fp64);
     if (rc) return rc;
   }
   if (!fp64) return density_list(h, with_pressure, vl, vcount, reuse ? h->vcap : h->neigh_cap);
@@ -1310,12 +1222,12 @@ int compute_force(Handle* h, int64_t step, int fuse_mode, double dt) {
     if (split)                                                                                   \
       k_force32<DD, NW, 4, ST><<<gp4, kReuseTPB, 0, s>>>(                                        \
           k, h->cell_start, h->cell_of, h->nl, h->ncount, h->neigh_cap, h->off, h->x, h->v,      \
-          h->pcf, h->vf, h->wd, h->f, h->st, fuse_mode, dt, h->v2, (uint32_t)step, step_ptr,     \
+          h->vf, h->wd, h->f, h->st, fuse_mode, dt, h->v2, (uint32_t)step, step_ptr,             \
           (float)inv_sqdt, h->d_err, nn, ca);                                                    \
     else                                                                                         \
       k_force32<DD, NW, 1, ST><<<gp, kReuseTPB, 0, s>>>(                                         \
           k, h->cell_start, h->cell_of, h->nl, h->ncount, h->neigh_cap, h->off, h->x, h->v,      \
-          h->pcf, h->vf, h->wd, h->f, h->st, fuse_mode, dt, h->v2, (uint32_t)step, step_ptr,     \
+          h->vf, h->wd, h->f, h->st, fuse_mode, dt, h->v2, (uint32_t)step, step_ptr,             \
           (float)inv_sqdt, h->d_err, nn, ca);                                                    \
   } while (0)
 #define PICK_F32_ST(DD, NW)                   \
@@ -1323,7 +1235,9 @@ int compute_force(Handle* h, int64_t step, int fuse_mode, double dt) {
     if (k.stress) LAUNCH_F32(DD, NW, true);   \
     else LAUNCH_F32(DD, NW, false);           \
   } while (0)
-    if (k.d == 3) {
+    if (force32_packed(h, (uint32_t)step, step_ptr, (float)inv_sqdt, fuse_mode, dt)) {
+      // done
+    } else if (k.d == 3) {
       if (k.newtonian) PICK_F32_ST(3, false); else PICK_F32_ST(3, true);
     } else {
       if (k.newtonian) PICK_F32_ST(2, false); else PICK_F32_ST(2, true);

@@ -67,13 +67,29 @@ __device__ __forceinline__ bool beyond(double d2, double rc2) {
   return b >= __double_as_longlong(rc2) && b <= 0x7ff0000000000000ll;
 }
 
-// FP32 -> FP64 on the integer pipe (exact; normal numbers and zero, which is
-// what Box-Muller with flush-to-zero gives)
+// FP32 -> FP64 on the integer pipe: exact for normal numbers; what is below
+// them (flushed to zero by the FP32 code) gives zero, infinity and NaN stay
+// non-finite
 __device__ __forceinline__ double widen(float z) {
   const unsigned u = __float_as_uint(z);
   const unsigned mag = u & 0x7fffffffu;
-  const unsigned hi = mag ? (u & 0x80000000u) | ((mag >> 3) + 0x38000000u) : 0u;
+  unsigned hi = (u & 0x80000000u) | ((mag >> 3) + 0x38000000u);
+  if (mag < 0x00800000u) return 0.0;
+  if (mag >= 0x7f800000u) hi |= 0x7ff00000u;
   return __hiloint2double((int)hi, (int)(u << 29));
+}
+
+// FP64 -> FP32 on the integer pipe, to nearest even; below FP32's normal numbers
+// zero (as flushed), above its range infinity, NaN stays NaN
+__device__ __forceinline__ float narrow(double z) {
+  const unsigned hi = (unsigned)__double2hiint(z), lo = (unsigned)__double2loint(z);
+  const unsigned mag = hi & 0x7fffffffu;
+  unsigned u = ((mag - 0x38000000u) << 3) | (lo >> 29);
+  const unsigned rest = lo << 3;  // the bits below, half an ulp at 0x80000000
+  u += (rest > 0x80000000u || (rest == 0x80000000u && (u & 1u))) ? 1u : 0u;
+  if (mag < 0x38100000u) u = 0u;
+  if (mag >= 0x47f00000u) u = (mag > 0x7ff00000u || (mag == 0x7ff00000u && lo)) ? 0x7fc00000u : 0x7f800000u;
+  return __uint_as_float(u | (hi & 0x80000000u));
 }
 
 // sqrt(a) and, with INV, 1/sqrt(a) from one seed: Goldschmidt's coupled

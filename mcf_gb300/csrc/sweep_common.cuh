@@ -83,8 +83,8 @@ __device__ __forceinline__ void write_particle_records(const Consts& k, int i, d
       q[i] = inv;
       for (int cc = 0; cc < d2; ++cc) q[(size_t)(1 + cc) * n + i] = k.G * nn.ct[(size_t)cc * n + i] * inv2;
     } else {
-      pcf[i] = make_float4((float)((p + k.G) * inv2), (float)inv2, (float)(1.0 / m), (float)p);
-      vf[i] = make_float4((float)v.x, (float)v.y, (float)v.z, __int_as_float(pid));
+      pcf[2 * i] = make_float4((float)((p + k.G) * inv2), (float)inv2, (float)(1.0 / m), (float)p);
+      vf[2 * i] = make_float4((float)v.x, (float)v.y, (float)v.z, __int_as_float(pid));
       float* q = (float*)nn.qq;
       q[i] = (float)inv;
       for (int cc = 0; cc < d2; ++cc)
@@ -98,18 +98,19 @@ __device__ __forceinline__ void write_particle_records(const Consts& k, int i, d
     pr[i] = p;
     pc[i] = pair_coeffs(k, rho, p, m);
   } else {
-    const float rf = (float)rho, mf = (float)m;
+    // conversions on the integer pipe (narrow, widen: the same roundings)
+    const float rf = narrow(rho), mf = narrow(m);
     const float r_eos = (k.rhs_density_type == 1) ? rf : rf * mf;
     float p;
     if (k.eos_type == 1) {
-      const float rg = (k.gamma == 1.0) ? r_eos : powf(r_eos, (float)k.gamma);
-      p = (float)k.c2 * (rg - (float)k.rho_ref);
+      const float rg = (k.gammaf == 1.0f) ? r_eos : powf(r_eos, k.gammaf);
+      p = k.c2f * (rg - k.rho_reff);
     } else {
-      const float q = r_eos / (float)k.rho_ref;
-      const float qg = (k.gamma == 1.0) ? q : powf(q, (float)k.gamma);
-      p = (float)k.p0 * (qg - 1.0f);
+      const float q = r_eos / k.rho_reff;
+      const float qg = (k.gammaf == 1.0f) ? q : powf(q, k.gammaf);
+      p = k.p0f * (qg - 1.0f);
     }
-    pr[i] = (double)p;
+    pr[i] = widen(p);
     const float inv = 1.0f / rf;
     float4 cc;
     switch (k.rhs_force_type) {
@@ -118,16 +119,111 @@ __device__ __forceinline__ void write_particle_records(const Consts& k, int i, d
       case 3: cc = make_float4(p * inv * inv, inv * inv, 1.0f / mf, p); break;
       default: cc = make_float4(p, inv * inv, 1.0f / mf, p); break;
     }
-    pcf[i] = cc;
-    vf[i] = make_float4((float)v.x, (float)v.y, (float)v.z, __int_as_float(pid));
+    pcf[2 * i] = cc;
+    vf[2 * i] = make_float4(narrow(v.x), narrow(v.y), narrow(v.z), __int_as_float(pid));
+  }
+}
+
+// A pair with a boundary particle, FP32 path: the wall or colloid particle
+// takes the no-slip velocity and the fluid partner's pressure (pp_interaction_
+// fw/wf/fc/cf.inc), in the Oldroyd-B model also its density and pressure
+// tensor.  Wall distances come from the FP64-rounded per-particle values (one
+// wall axis) or from the FP64 positions (several).  ci_w, cj_w: the two
+// pressures; qi is particle i's polymer record, qie / qj those of the pair.
+template <int D, bool NNW>
+__device__ __forceinline__ void boundary_pair32(const Consts& k, int i, int j, int si, int sj,
+                                                const float* r, float2 wdi,
+                                                const float2* __restrict__ wd,
+                                                const double4_32a* __restrict__ x,
+                                                const CollArgs& ca, float ci_w, float cj_w,
+                                                float* vi, float* vj, float& Ai, float& Aj,
+                                                float& Bi, float& Bj, const float* qi, float* qie,
+                                                float* qj) {
+  constexpr int D2 = D * D;
+  const bool other_j = (si < 0 || sj < 0) ? sj < 0 : sj > 0;  // the boundary particle is j
+  float vw[3];
+  bool noslip = true;
+  if (si < 0 || sj < 0) {
+    const int sw = (sj < 0) ? sj : si;
+    const int face = -sw;
+    const bool lower = (face & 1) != 0;
+    float df, dw;
+    if (k.wall_axis >= 0) {
+      const float2 wj = wd[j];
+      const float di = lower ? wdi.x : wdi.y, dj = lower ? wj.x : wj.y;
+      df = (sj < 0) ? di : dj;
+      dw = (sj < 0) ? dj : di;
+    } else {
+      const int axis = (face - 1) >> 1;
+      const double x_sur = axis == 0 ? (lower ? k.min_phys[0] : k.max_phys[0])
+                           : axis == 1 ? (lower ? k.min_phys[1] : k.max_phys[1])
+                                       : (lower ? k.min_phys[2] : k.max_phys[2]);
+      const double4_32a a4 = x[i], b4 = x[j];
+      const double xa = axis == 0 ? a4.x : axis == 1 ? a4.y : a4.z;
+      const double xb = axis == 0 ? b4.x : axis == 1 ? b4.y : b4.z;
+      df = (float)(((sj < 0) ? xa : xb) - x_sur);
+      dw = (float)(((sj < 0) ? xb : xa) - x_sur);
+    }
+    if (other_j)
+      wall_noslip_dist<float, D>(k, df, dw, vi, sj, vw);
+    else
+      wall_noslip_dist<float, D>(k, df, dw, vj, si, vw);
+  } else if (k.coll_noslip == 2) {
+    const float4 rc4 = ca.rxcf[other_j ? j : i];
+    const float rxc_[3] = {rc4.x, rc4.y, rc4.z};
+    if (other_j) {
+      colloid_noslip<float, D>(k, sj - 1, rxc_, r, vi, vw);
+    } else {
+      const float rfc[3] = {-r[0], -r[1], -r[2]};
+      colloid_noslip<float, D>(k, si - 1, rxc_, rfc, vj, vw);
+    }
+  } else {
+    noslip = false;  // frozen: the boundary particle's own (rigid) velocity
+  }
+  if (other_j) {
+    if (noslip)
+#pragma unroll
+      for (int a = 0; a < D; ++a) vj[a] = vw[a];
+    if (NNW) {
+      Aj = Ai;
+      Bj = Bi;
+#pragma unroll
+      for (int cc = 0; cc <= D2; ++cc) qj[cc] = qi[cc];
+    } else {
+      Aj = boundary_A<float>(k.rhs_force_type, ci_w, Bj);
+    }
+  } else {
+    if (noslip)
+#pragma unroll
+      for (int a = 0; a < D; ++a) vi[a] = vw[a];
+    if (NNW) {
+      Ai = Aj;
+      Bi = Bj;
+#pragma unroll
+      for (int cc = 0; cc <= D2; ++cc) qie[cc] = qj[cc];
+    } else {
+      Ai = boundary_A<float>(k.rhs_force_type, cj_w, Bi);
+    }
   }
 }
 
 constexpr int kReuseTPB = 128;
-// below this many particles the FP32 force sweep runs 4 lanes per particle
+// below this many particles the scalar FP32 force sweep and the FP64 density
+// run 4 lanes per particle
 constexpr int64_t kSplitBelow = 50000;
 // and below this many the FP64 density sweep runs 8
 constexpr int64_t kSplit8Below = 12000;
+// Lanes per particle of the packed FP32 sweeps: a lane takes whole octets of a
+// list, and a 2D particle has about four octets of pairs, a 3D one fourteen or
+// more.  Measured, us a step (lanes 16 / 4 / 1): 3D rc = 3 dx 6k particles 66 /
+// 84 / 191, 18k 114 / 91 / 170, 41k 189 / 150 / 185, 71k 296 / 194 / 206, 91k 350 /
+// 222 / 187; 3D rc = 4 dx 8k 76 / 84 / 226, 33k 201 / 139 / 211, 91k 503 / 328 / 342;
+// 2D 10k 59 / 36 / 46, 23k 87 / 49 / 47, 63k 188 / 77 / 55.
+constexpr int64_t kLanes16Below = 12000, kLanes4Below = 75000, kLanes4Below2D = 20000;
+inline int lanes32(int64_t n, int dim) {
+  if (dim == 2) return n < kLanes4Below2D ? 4 : 1;
+  return n < kLanes16Below ? 16 : n < kLanes4Below ? 4 : 1;
+}
 
 // FP32 offset of each stencil slot (the neighbour cell's origin minus the
 // home cell's, w = Lees-Edwards velocity jump), build_table's t.o, in a
@@ -142,11 +238,32 @@ __device__ __forceinline__ void fill_slot_offsets(const Consts& k, float4* s_slo
   if (e < kSlotTable) s_slot[e] = slot_offset<D>(k, e % kMaxStencil, e / kMaxStencil);
 }
 
-// Physical list row of logical entry p of a list in two segments: entries
-// below nff from row 0 up, the others from row cap-1 down (the FP32
-// candidate and pair lists; an unsplit list has nff = its count).
-__device__ __forceinline__ int cand_row(int p, int nff, int cap) {
-  return p < nff ? p : cap - 1 - (p - nff);
+// One partner's FP32 records: offset to its cell's origin (w = species id),
+// velocity (w = pid bits) and pair coefficients (A, B, C, p), and its slot.
+struct JData {
+  float4 o, v, c;
+  int sl, j;
+};
+
+// the velocity and coefficient records lie side by side (one 32-byte load)
+__device__ __forceinline__ void load_vc(const float4* __restrict__ vf, int j, float4& v,
+                                        float4& c) {
+  const double4_32a t = *(reinterpret_cast<const double4_32a*>(vf) + j);
+  v = make_float4(__int_as_float(__double2loint(t.x)), __int_as_float(__double2hiint(t.x)),
+                  __int_as_float(__double2loint(t.y)), __int_as_float(__double2hiint(t.y)));
+  c = make_float4(__int_as_float(__double2loint(t.z)), __int_as_float(__double2hiint(t.z)),
+                  __int_as_float(__double2loint(t.w)), __int_as_float(__double2hiint(t.w)));
+}
+
+__device__ __forceinline__ JData load_j(const int* __restrict__ s_start, int ent,
+                                        const float4* __restrict__ off,
+                                        const float4* __restrict__ vf) {
+  JData d;
+  d.sl = ent >> kLocalBits;
+  d.j = s_start[d.sl * kReuseTPB + threadIdx.x] + (ent & (kMaxCellCount - 1));
+  d.o = off[d.j];
+  load_vc(vf, d.j, d.v, d.c);
+  return d;
 }
 
 // slot offsets of the Lees-Edwards row state of the home cell

@@ -343,6 +343,9 @@ __global__ void k_colloid_follow(Consts k, const int* __restrict__ cstart,
       cd[3 + i] = (i < D) ? r[kRecV + i] : 0.0;
       cd[6 + i] = r[kRecOm + i];
     }
+    float* cf = k.collf + (size_t)c * 12;  // the FP32 copy
+#pragma unroll
+    for (int i = 0; i < 9; ++i) cf[i] = narrow(cd[i]);
   }
 }
 

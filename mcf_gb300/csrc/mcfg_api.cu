@@ -177,6 +177,7 @@ void free_all(Handle* h) {
   h->rxc = nullptr;
   h->rxcf = nullptr;
   h->k.coll = nullptr;
+  h->k.collf = nullptr;
   h->k.ncoll = 0;
   h->off = h->pcf = h->vf = nullptr;
   h->wd = nullptr;
@@ -340,6 +341,7 @@ void make_consts(const mcfg_params& p, Consts& k) {
   k.eta_coef = p.eta_coef;
   k.kt = p.kt;
   k.machine_zero = 1e-14;  // technique_new.F90:361-363
+  k.machine_zerof = (float)k.machine_zero;
   k.noise = (p.Brownian && p.kt > k.machine_zero) ? 1 : 0;
   k.wall_rho_type = p.wall_rho_type;
   k.wall_noslip_type = p.wall_noslip_type;
@@ -1671,7 +1673,7 @@ static int put_colloid_state(Handle* h, int nc, const double* x, const double* v
   h->cx.assign(x, x + (size_t)nc * d);
   h->cv.assign(v, v + (size_t)nc * d);
   h->com.assign(omega, omega + (size_t)nc * 3);
-  std::vector<double> buf((size_t)nc * 12, 0.0);
+  std::vector<double> buf((size_t)nc * 18, 0.0);
   for (int c = 0; c < nc; ++c) {
     for (int a = 0; a < d; ++a) {
       buf[(size_t)c * 12 + a] = x[(size_t)c * d + a];
@@ -1680,6 +1682,9 @@ static int put_colloid_state(Handle* h, int nc, const double* x, const double* v
     for (int a = 0; a < 3; ++a) buf[(size_t)c * 12 + 6 + a] = omega[(size_t)c * 3 + a];
     buf[(size_t)c * 12 + 9] = h->crad[(size_t)c];
   }
+  // the FP32 copy behind it
+  float* bf = reinterpret_cast<float*>(buf.data() + (size_t)nc * 12);
+  for (size_t q = 0; q < (size_t)nc * 12; ++q) bf[q] = (float)buf[q];
   if (nc > 0 &&
       (cuda_check(h, cudaMemcpyAsync(h->coll, buf.data(), sizeof(double) * buf.size(),
                                      cudaMemcpyHostToDevice, h->stream), "upload colloids") ||
@@ -1709,7 +1714,7 @@ int mcfg_set_colloids(mcfg_handle* h, const mcfg_colloid_params* cp, const doubl
   h->crad.assign(radius, radius + nc);
   if (nc > 0) {
     int rc;
-    if ((rc = dalloc(h, &h->coll, (size_t)nc * 12)) ||
+    if ((rc = dalloc(h, &h->coll, (size_t)nc * 18)) ||
         (rc = dalloc(h, &h->coll_out, (size_t)nc * 12)))
       return rc;
   }
@@ -1717,6 +1722,7 @@ int mcfg_set_colloids(mcfg_handle* h, const mcfg_colloid_params* cp, const doubl
   Consts& k = h->k;
   k.ncoll = nc;
   k.coll = h->coll;
+  k.collf = reinterpret_cast<float*>(h->coll + (size_t)nc * 12);
   k.coll_noslip = cp->noslip_type;
   k.coll_rho_type = cp->rho_type;
   k.coll_translate = cp->translate;

@@ -103,6 +103,8 @@ struct Consts {
   int ncoll, coll_noslip, coll_rho_type, coll_translate, coll_rotate, pp_cc;
   double coll_dout;
   const double* coll;    // device [ncoll][12]: X(3) V(3) Omega(3) R pad(2)
+  float* collf;          // the same in FP32, behind it (the FP32 pair terms read it:
+                         // a conversion is an FP64 instruction a pair)
   // Oldroyd-B conformation model (Newtonian == 0)
   int newtonian;
   double G, tau, inv_tau;  // G = n_p kt_p
@@ -112,6 +114,7 @@ struct Consts {
   int body_force_type;
   double body_force[3];
   double machine_zero;
+  float machine_zerof;
 };
 
 struct Handle {
@@ -175,7 +178,7 @@ struct Handle {
   // colloids
   mcfg_colloid_params cp{};
   std::vector<double> cx, cv, com, crad;  // host copies (repulsion)
-  double* coll = nullptr;      // device [nc][12]
+  double* coll = nullptr;      // device [nc][12], then the same in float
   int* coll_start = nullptr;   // [nc+1] CSR of boundary particles (host indices)
   int* coll_mem = nullptr;
   int coll_nmem = 0;

@@ -37,6 +37,7 @@ struct KC<double> {
   __device__ static double coef_grad(const Consts& k) { return k.coef_grad; }
   __device__ static double eta(const Consts& k) { return k.eta; }
   __device__ static double kt(const Consts& k) { return k.kt; }
+  __device__ static double zero(const Consts& k) { return k.machine_zero; }
   __device__ static double eta_coef(const Consts& k) { return k.eta_coef; }
 };
 template <>
@@ -47,6 +48,7 @@ struct KC<float> {
   __device__ static float coef_grad(const Consts& k) { return k.coef_gradf; }
   __device__ static float eta(const Consts& k) { return k.etaf; }
   __device__ static float kt(const Consts& k) { return k.ktf; }
+  __device__ static float zero(const Consts& k) { return k.machine_zerof; }
   __device__ static float eta_coef(const Consts& k) { return k.eta_coeff; }
 };
 
@@ -606,10 +608,14 @@ __device__ __forceinline__ void cross3t(const T* a, const T* b, T* o) {
 template <typename T, int D>
 __device__ __forceinline__ void colloid_noslip(const Consts& k, int c, const T* r_xc,
                                                const T* r_fc, const T* vf, T* vc) {
-  const double* cd = k.coll + (size_t)c * 12;
-  const T R = (T)cd[9];
-  T V[3] = {(T)cd[3], (T)cd[4], (T)cd[5]};
-  const T om[3] = {(T)cd[6], (T)cd[7], (T)cd[8]};
+  const T* cd;  // the table in T
+  if constexpr (std::is_same<T, double>::value)
+    cd = k.coll + (size_t)c * 12;
+  else
+    cd = k.collf + (size_t)c * 12;
+  const T R = cd[9];
+  T V[3] = {cd[3], cd[4], cd[5]};
+  const T om[3] = {cd[6], cd[7], cd[8]};
   T r_xf[3] = {0, 0, 0};
   T dd = 0;
 #pragma unroll
@@ -634,7 +640,7 @@ __device__ __forceinline__ void colloid_noslip(const Consts& k, int c, const T* 
   const T d_cs = R - d_cn;
   const T d_fs = d_fcoll - R;
   T corr;
-  if (fabs(d_fs) < (T)k.machine_zero) {
+  if (fabs(d_fs) < KC<T>::zero(k)) {
     corr = T(0.5);  // mcf_colloid_dist_ratio_max
   } else {
     corr = d_cs / d_fs;

@@ -361,9 +361,21 @@ __global__ void k_pressure(Consts k, const double* __restrict__ rho, const doubl
 }
 
 // ---------------------------------------------------------------------------
-// FP64 force sweep
+// FP64 force sweep: Oldroyd-B, stress, colloids, Lees-Edwards (k_force_sym has
+// the rest).  S lanes per particle take every S-th entry, as in
+// k_density_reuse; their sums are added in lane order.  9,216 2D Oldroyd-B particles (288 warps for 608
+// schedulers with one lane each): the adjoint of 20 steps 9.3 -> 7.6 ms.
 // ---------------------------------------------------------------------------
-template <int D, bool NNW>
+template <int S>
+__device__ __forceinline__ double lane_sum(double part, unsigned gmask) {
+  const int base = (threadIdx.x & 31) & ~(S - 1);
+  double tot = __shfl_sync(gmask, part, base);
+#pragma unroll
+  for (int q = 1; q < S; ++q) tot += __shfl_sync(gmask, part, base + q);
+  return tot;
+}
+
+template <int D, bool NNW, int S>
 __global__ void __launch_bounds__(kReuseTPB)
     k_force64(Consts k, const int* __restrict__ cell_start, const int* __restrict__ cell_of,
               const uint16_t* __restrict__ nl,
@@ -383,8 +395,9 @@ __global__ void __launch_bounds__(kReuseTPB)
   __shared__ int s_shift[kMaxStencil * kReuseTPB];
   const int n = k.n;
   const bool noise = k.noise != 0;
-  const int i = blockIdx.x * kReuseTPB + threadIdx.x;
-  if (i >= n) return;
+  const int gt = blockIdx.x * kReuseTPB + threadIdx.x;
+  const int i = gt / S, lane_s = gt % S;
+  if (i >= n) return;  // the S lanes of a particle leave together
   build_lane_table<D, kReuseTPB>(k, cell_of[i], cell_start, s_start, s_shift);
   const int si = sid[i];
   const int pidi = pid[i];
@@ -406,7 +419,7 @@ __global__ void __launch_bounds__(kReuseTPB)
 #pragma unroll
   for (int a = 0; a < 9; ++a) sacc[a] = 0;
   const int cnt = ncount[i];
-  for (int e = 0; e < cnt; ++e) {
+  for (int e = lane_s; e < cnt; e += S) {
     const int ent = nl[up_at(e, n, i)];
     const int sl = ent >> kLocalBits, q = ent & (kMaxCellCount - 1);
     const int j = s_start[sl * kReuseTPB + threadIdx.x] + q;
@@ -550,6 +563,20 @@ __global__ void __launch_bounds__(kReuseTPB)
 #pragma unroll
         for (int a = 0; a < D; ++a) sacc[b * D + a] += r[a] * pa[b] * T(0.5);
     }
+  }
+  if (S > 1) {
+    const unsigned gmask = group_mask<S>();
+#pragma unroll
+    for (int a = 0; a < D; ++a) acc[a] = lane_sum<S>(acc[a], gmask);
+    if (nnw) {
+#pragma unroll
+      for (int cc = 0; cc < D2; ++cc) L[cc] = lane_sum<S>(L[cc], gmask);
+    }
+    if (k.stress) {
+#pragma unroll
+      for (int a = 0; a < D2; ++a) sacc[a] = lane_sum<S>(sacc[a], gmask);
+    }
+    if (lane_s != 0) return;
   }
   if (k.stress) {
 #pragma unroll
@@ -1205,16 +1232,22 @@ int compute_force(Handle* h, int64_t step, int fuse_mode, double dt) {
 #undef LAUNCH_SYM
     h->launches++;
   } else if (fp64) {
-#define LAUNCH_F64(DD, NW)                                                                      \
-  k_force64<DD, NW><<<gp, kReuseTPB, 0, s>>>(k, h->cell_start, h->cell_of, h->nl, h->ncount,     \
-                                            h->x, h->v, h->pc,                                 \
-                                     h->sid, h->pid, h->f, h->st, fuse_mode, dt, h->v2,          \
-                                     (uint32_t)step, step_ptr, inv_sqdt, h->d_err, nn, ca)
+#define LAUNCH_F64(DD, NW, SS)                                                                   \
+  k_force64<DD, NW, SS><<<std::max(1, (int)((h->n * SS + kReuseTPB - 1) / kReuseTPB)), kReuseTPB, \
+                          0, s>>>(k, h->cell_start, h->cell_of, h->nl, h->ncount, h->x, h->v,    \
+                                  h->pc, h->sid, h->pid, h->f, h->st, fuse_mode, dt, h->v2,      \
+                                  (uint32_t)step, step_ptr, inv_sqdt, h->d_err, nn, ca)
+#define PICK_F64(DD, NW)               \
+  do {                                 \
+    if (split) LAUNCH_F64(DD, NW, 4);  \
+    else LAUNCH_F64(DD, NW, 1);        \
+  } while (0)
     if (k.d == 3) {
-      if (k.newtonian) LAUNCH_F64(3, false); else LAUNCH_F64(3, true);
+      if (k.newtonian) PICK_F64(3, false); else PICK_F64(3, true);
     } else {
-      if (k.newtonian) LAUNCH_F64(2, false); else LAUNCH_F64(2, true);
+      if (k.newtonian) PICK_F64(2, false); else PICK_F64(2, true);
     }
+#undef PICK_F64
 #undef LAUNCH_F64
   } else {
 #define LAUNCH_F32(DD, NW, ST)                                                                  \

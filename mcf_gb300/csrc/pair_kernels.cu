@@ -794,25 +794,28 @@ __global__ void __launch_bounds__(kReuseTPB, (NNW && D == 3) ? 4 : 5)
 // Bound: the FP64 pipe (84% busy); what counts is FP64 slots a pair.  Runs of
 // 4 spread the owner reduction (15 adds + 3) over 128 pairs; the mass factor
 // is left to the gather (not for the Morris form, whose factor is the
-// partner's mass).  64^3 with noise: 2.64 ms, 86 slots
+// partner's mass).  COOP: a block's warps share one cell, for systems with few
+// cells (kCoopCells).  64^3 with noise: 2.64 ms, 86 slots
 // a pair, against 3.02 ms and 100 with one pair a round and lane.
 // ---------------------------------------------------------------------------
-constexpr int kSymCC = 32;  // partners per slot held in shared memory
-constexpr int kRun = 4;     // consecutive pairs a lane takes in a round
+// partners per slot held in shared memory (a fuller cell's sums lie in global
+// memory): systems with few cells can afford more
+template <int D, bool COOP>
+constexpr int kSymCC = (D == 3 && COOP) ? 64 : 32;
 
 // Per-warp dynamic shared memory of k_force_sym (bytes):
 // part[NSF][D][CC] | acc[D][32] | ex[33] e0[32] pad | x v pc [32] sid pid [32]
-template <int D>
+template <int D, bool COOP>
 __host__ __device__ constexpr int sym_warp_bytes() {
   constexpr int NSF = (D == 3) ? 14 : 5;
-  constexpr int part = NSF * D * kSymCC * 8;
+  constexpr int part = NSF * D * kSymCC<D, COOP> * 8;
   constexpr int acc = D * 32 * 8;
   constexpr int idx = 96 * 4;
   constexpr int own = 3 * 32 * 32 + 2 * 32 * 4;
   return (part + acc + idx + own + 31) / 32 * 32;
 }
 
-template <int D>
+template <int D, bool COOP>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     k_force_sym(Consts k, const int* __restrict__ cell_start, const uint16_t* __restrict__ nl,
                 const int* __restrict__ ncount, const int* __restrict__ nhs,
@@ -823,13 +826,14 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   // the Philox counter's step: the argument, or the device step counter
   // when the sweep runs inside a captured graph
   const uint32_t step = step_ptr ? (uint32_t)*step_ptr : step_arg;
-  constexpr int CC = kSymCC;
+  constexpr int CC = kSymCC<D, COOP>;
+  constexpr int kRun = (COOP && D == 2) ? 1 : 4;  // consecutive pairs a lane takes in a round
   constexpr int CENTER = (D == 3) ? 13 : 4;
   constexpr int NSF = (D == 3) ? 14 : 5;  // forward slots CENTER..NS-1
   extern __shared__ __align__(32) unsigned char smem_raw[];
   __shared__ NbTable tab[kWarpsPerBlock];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned char* wb = smem_raw + (size_t)wib * sym_warp_bytes<D>();
+  unsigned char* wb = smem_raw + (size_t)wib * sym_warp_bytes<D, COOP>();
   double* part = reinterpret_cast<double*>(wb);
   double* acc_s = part + NSF * D * CC;
   int* ex = reinterpret_cast<int*>(acc_s + D * 32);
@@ -839,10 +843,15 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   const int n = k.n;
   const bool noise = k.noise != 0;
   const bool scaled = k.rhs_force_type == 1;
-  for (int cell = blockIdx.x * kWarpsPerBlock + wib; cell <= k.ncell;
-       cell += gridDim.x * kWarpsPerBlock) {
+  for (int cell = COOP ? blockIdx.x : blockIdx.x * kWarpsPerBlock + wib; cell <= k.ncell;
+       cell += gridDim.x * (COOP ? 1 : kWarpsPerBlock)) {
     NbTable& t = tab[wib];
     build_table<D>(k, cell, cell_start, t);
+    // shared cells: the warps take rounds in turn, each with sums of its own;
+    // sums in global memory (a neighbour cell of more than CC) have one writer
+    bool solo = false;
+    if (COOP)
+      for (int s = 0; s < NSF; ++s) solo = solo || t.count[CENTER + s] > CC;
     // zero the partner sums this cell owns (shared, or global when a cell
     // holds more than CC particles)
     for (int s = 0; s < NSF; ++s) {
@@ -852,7 +861,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
         for (int a = 0; a < D; ++a) {
           if (cs_ <= CC)
             part[(s * D + a) * CC + q] = 0.0;
-          else
+          else if (!COOP || wib == 0)
             jp[((size_t)s * D + a) * n + st_ + q] = 0.0;
         }
     }
@@ -884,7 +893,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
       e0s[lane] = e0;
       if (lane == 31) ex[32] = total;
       __syncwarp();
-      for (int r0 = 0; r0 < total; r0 += 32 * kRun) {
+      const int turns = (COOP && !solo) ? kWarpsPerBlock : 1;
+      const int mine = COOP && solo && wib > 0 ? 0 : total;
+      for (int r0 = (turns > 1 ? wib : 0) * 32 * kRun; r0 < mine; r0 += turns * 32 * kRun) {
         // the run's first pair and its owner
         int fidx = r0 + lane * kRun;
         int ow_l = 0;
@@ -1022,22 +1033,44 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
         }
         __syncwarp();
       }
-      if (act) {
+      // this warp's sums, or in a shared cell all warps' in warp order
+      constexpr int kHop = sym_warp_bytes<D, COOP>() / 8;
+      if (COOP) __syncthreads();
+      if (act && (!COOP || wib == 0)) {
 #pragma unroll
-        for (int a = 0; a < D; ++a) jp[((size_t)NSF * D + a) * n + i] = acc_s[a * 32 + lane];
+        for (int a = 0; a < D; ++a) {
+          double sum = acc_s[a * 32 + lane];
+          if (COOP)
+#pragma unroll
+            for (int w = 1; w < kWarpsPerBlock; ++w) sum += acc_s[w * kHop + a * 32 + lane];
+          jp[((size_t)NSF * D + a) * n + i] = sum;
+        }
       }
-      __syncwarp();
+      if (COOP)
+        __syncthreads();
+      else
+        __syncwarp();
     }
+    constexpr int kHop = sym_warp_bytes<D, COOP>() / 8;
+    const double* part0 = COOP ? reinterpret_cast<const double*>(smem_raw) : part;
     __syncwarp();
-    for (int s = 0; s < NSF; ++s) {
+    for (int s = COOP ? wib : 0; s < NSF; s += COOP ? kWarpsPerBlock : 1) {
       const int cs_ = t.count[CENTER + s], st_ = t.start[CENTER + s];
       if (cs_ > CC) continue;
       for (int q = lane; q < cs_; q += 32)
 #pragma unroll
-        for (int a = 0; a < D; ++a)
-          jp[((size_t)s * D + a) * n + st_ + q] = part[(s * D + a) * CC + q];
+        for (int a = 0; a < D; ++a) {
+          double sum = part0[(s * D + a) * CC + q];
+          if (COOP)
+#pragma unroll
+            for (int w = 1; w < kWarpsPerBlock; ++w) sum += part0[w * kHop + (s * D + a) * CC + q];
+          jp[((size_t)s * D + a) * n + st_ + q] = sum;
+        }
     }
-    __syncwarp();
+    if (COOP)
+      __syncthreads();
+    else
+      __syncwarp();
   }
 }
 
@@ -1194,6 +1227,11 @@ int compute_pressure(Handle* h) {
   return MCFG_OK;
 }
 
+// below this many cells the symmetric sweep's warps share cells
+// (us a step, own cells / shared: 3D 100 cells 719 / 235, 1,000 896 / 729, 4,913
+// 2664 / 2612, 9,261 4446 / 4558; 2D 441 cells 69 / 54, 9,801 350 / 349)
+constexpr int kCoopCells = 6000;
+
 int compute_force(Handle* h, int64_t step, int fuse_mode, double dt) {
   Consts& k = h->k;
   cudaStream_t s = h->stream;
@@ -1217,18 +1255,24 @@ int compute_force(Handle* h, int64_t step, int fuse_mode, double dt) {
     const int gbn = (n + 255) / 256;
     double* jp = (double*)h->jp;
     // the attribute is per device: set it for the handle's (a host call)
-#define LAUNCH_SYM(DD)                                                                           \
+#define LAUNCH_SYM(DD, CO)                                                                       \
   do {                                                                                           \
-    constexpr int bytes = kWarpsPerBlock * sym_warp_bytes<DD>();                                 \
-    cudaFuncSetAttribute(k_force_sym<DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);   \
-    k_force_sym<DD><<<g, bs, bytes, s>>>(k, h->cell_start, h->nl, h->ncount, h->nhs, h->x, h->v, \
-                                         h->pc, h->sid, h->pid, jp, (uint32_t)step, step_ptr,    \
-                                         inv_sqdt);                                              \
+    constexpr int bytes = kWarpsPerBlock * sym_warp_bytes<DD, CO>();                                 \
+    cudaFuncSetAttribute(k_force_sym<DD, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
+                         bytes);                                                                 \
+    k_force_sym<DD, CO><<<CO ? k.ncell + 1 : g, bs, bytes, s>>>(                                 \
+        k, h->cell_start, h->nl, h->ncount, h->nhs, h->x, h->v, h->pc, h->sid, h->pid, jp,       \
+        (uint32_t)step, step_ptr, inv_sqdt);                                                     \
     if (n > 0)                                                                                   \
       k_force_gather<DD><<<gbn, 256, 0, s>>>(k, h->cell_of, jp, h->x, h->v, h->pc, h->sid, h->f, \
                                              fuse_mode, dt, h->v2, h->d_err);                    \
   } while (0)
-    if (k.d == 3) LAUNCH_SYM(3); else LAUNCH_SYM(2);
+    const bool coop = k.ncell < kCoopCells;
+    if (k.d == 3) {
+      if (coop) LAUNCH_SYM(3, true); else LAUNCH_SYM(3, false);
+    } else {
+      if (coop) LAUNCH_SYM(2, true); else LAUNCH_SYM(2, false);
+    }
 #undef LAUNCH_SYM
     h->launches++;
   } else if (fp64) {

@@ -64,3 +64,41 @@ def test_coincident_particles(dim):
     assert np.abs(g.download("rho")["rho"] / (2 * 66.0 * coef) - 1.0).max() <= 16 * EPS
     with pytest.raises(MCFGError, match="non-finite"):
         g.marching_init_force(0)
+
+
+def _forces(p, x, v, m, ids):
+    from oracle.oracle import Oracle
+    g, o = SDPD(p), Oracle(p)
+    for side in (g, o):
+        side.upload(x, v, m, ids)
+        side.marching_init_force(0)
+    a, b = g.download("f")["f"], o.download("f")["f"]
+    # the FP64 path's acceleration bar, with its floor of 1e-6 of the median scale
+    scale = o.force_scale()
+    scale = np.maximum(scale, 1e-6 * np.median(scale))[:, None] + np.abs(b)
+    assert (np.abs(a - b) <= 1e-12 * scale).all()
+
+
+@pytest.mark.parametrize("form", [1, 3])
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("crowd", [1, 32, 33, 64, 65, 150])
+def test_symmetric_sweep_crowded_cells(crowd, dim, form):
+    # partner sums in shared or global memory, more than one chunk of owners
+    rng = np.random.default_rng(crowd)
+    p, _, _, _, _ = _pair(dim, 1.0, rhs_force_type=form, rhs_density_type=1 if form == 1 else 2)
+    p.reserved[0] = 512
+    x = np.concatenate([rng.uniform(0.05, 2.9, (crowd, dim)),
+                        np.r_[3.1, 0.05, 0.05][:dim] + rng.uniform(0.0, 2.8, (crowd, dim)),
+                        rng.uniform(0.0, 12.0, (40, dim))])
+    n = len(x)
+    ids = np.stack([np.arange(1, n + 1), np.zeros(n)], axis=1).astype(np.int32)
+    _forces(p, x, rng.normal(0.0, 0.1, (n, dim)), np.ones(n), ids)
+
+
+@pytest.mark.parametrize("side", [55, 58])
+def test_symmetric_sweep_shared_cells_threshold(side):
+    # 5,832 and 6,859 cells: a cell to a block, a cell to a warp
+    from mcf_gb300 import configs
+    w = configs.c2_fluctuating_3d(n_side=side)
+    w.params.Brownian, w.params.kt = 0, 0.0
+    _forces(w.params, w.x, w.v, w.m, w.id)

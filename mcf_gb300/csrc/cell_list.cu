@@ -170,7 +170,7 @@ __global__ void k_cell_finalize(Consts k, const int* __restrict__ start,
     for (int a = 0; a < D; ++a) {
       const int ca = c % k.nm[a];
       c /= k.nm[a];
-      org[a] = k.xmin[a] + (double)ca * k.cs[a];
+      org[a] = k.org[a * k.org_pitch + ca];
     }
   }
   for (int e = lane; e < cnt; e += 32) {
@@ -221,7 +221,7 @@ __global__ void k_zero_counts(int* __restrict__ cnt, int nbins, const int* __res
 
 // after a gated rebuild: the permuted state back into the primary buffers
 // (a host-side pointer swap cannot depend on the device flag) and the
-// reference positions of the new candidate list
+// reference offsets of the new candidate list
 template <int D>
 __global__ void k_copy_back(int n, const int* __restrict__ gate, const double4_32a* __restrict__ x2,
                             const double4_32a* __restrict__ v2, const double4_32a* __restrict__ f2,
@@ -232,13 +232,15 @@ __global__ void k_copy_back(int n, const int* __restrict__ gate, const double4_3
                             double4_32a* __restrict__ f, double* __restrict__ m,
                             int* __restrict__ pid, int* __restrict__ sid, int* __restrict__ hidx,
                             double* __restrict__ ct, double* __restrict__ act,
-                            double4_32a* __restrict__ x_ref) {
+                            const float4* __restrict__ off, double y0,
+                            float4* __restrict__ off_ref) {
   if (*gate == 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double4_32a xp = x2[i];
   x[i] = xp;
-  x_ref[i] = xp;
+  const float4 of = off[i];
+  off_ref[i] = make_float4(of.x, of.y, of.z, (float)(xp.y - y0));
   v[i] = v2[i];
   f[i] = f2[i];
   m[i] = m2[i];
@@ -312,7 +314,7 @@ static int cell_list_launches(Handle* h, const int* gate) {
 #define COPY_BACK(DD)                                                                            \
   k_copy_back<DD><<<gb, tb, 0, s>>>(n, gate, h->x2, h->v2, h->f2, h->m2, h->pid2, h->sid2,       \
                                     h->hidx2, h->ct2, h->act2, h->x, h->v, h->f, h->m, h->pid,   \
-                                    h->sid, h->hidx, h->ct, h->act, h->x_ref)
+                                    h->sid, h->hidx, h->ct, h->act, h->off, k.le_y0, h->off_ref)
       if (k.d == 3) COPY_BACK(3); else COPY_BACK(2);
 #undef COPY_BACK
       h->launches++;

@@ -145,9 +145,11 @@ void free_all(Handle* h) {
   h->out_dev = nullptr;
   h->out_host = nullptr;
   h->out_cap = 0;
-  for (void* p : {(void*)h->x_ref, (void*)h->vl, (void*)h->vcount, (void*)h->d_rebuild})
+  for (void* p : {(void*)h->off_ref, (void*)h->org, (void*)h->vl, (void*)h->vcount, (void*)h->d_rebuild})
     if (p) cudaFree(p);
-  h->x_ref = nullptr;
+  h->off_ref = nullptr;
+  h->org = nullptr;
+  h->k.org = nullptr;
   h->vl = nullptr;
   h->vcount = h->d_rebuild = nullptr;
   h->vcap = 0;
@@ -248,6 +250,16 @@ namespace {
 
 namespace mcfg {
 
+// The rebuild test runs in FP32 on cell offsets: each is rounded (6e-8 of a
+// cell side), so the bound on their difference is drawn in by more than two
+// such roundings an axis can make (and, sheared, by that of y_ref le_aff).
+void far_bound(Consts& k, double half) {
+  double side = 0.0;
+  for (int a = 0; a < k.d; ++a) side = std::max(side, k.cs[a]);
+  const double b = std::max(0.0, half - 4e-7 * side - 2e-7 * std::fabs(k.le_aff) * k.len[1]);
+  k.far2f = (float)(b * b * (1.0 - 1e-6));
+}
+
 void make_consts(const mcfg_params& p, Consts& k) {
   memset(&k, 0, sizeof k);
   k.d = p.num_dim;
@@ -294,9 +306,9 @@ void make_consts(const mcfg_params& p, Consts& k) {
     if (skin > 0.0) {
       k.reuse = 1;
       k.half_skin2 = 0.25 * skin * skin;
-      k.half_skin_le2 = k.half_skin2;
       const double rv = p.cut_off + skin;
       k.rv2f = (float)(rv * rv * (1.0 + 1e-4));
+      far_bound(k, 0.5 * skin);
     }
   }
   // FP32 prefilter of the FP64 path: relative slack far above the FP32
@@ -365,7 +377,11 @@ void make_consts(const mcfg_params& p, Consts& k) {
     k.rk[2 * r + 1] = k.key1 + (uint32_t)r * 0xBB67AE85u;
   }
   k.body_force_type = p.body_force_type;
-  for (int a = 0; a < 3; ++a) k.body_force[a] = p.body_force[a];
+  k.body_on = 0;
+  for (int a = 0; a < 3; ++a) {
+    k.body_force[a] = p.body_force[a];
+    if (std::fabs(p.body_force[a]) > k.machine_zero) k.body_on |= 1 << a;
+  }
 }
 
 }  // namespace mcfg
@@ -377,6 +393,13 @@ void fill_consts(Handle* h) {
   h->le_skin = h->k.reuse ? 2.0 * std::sqrt(h->k.half_skin2) : 0.0;
   h->le_reach = h->p.cut_off + h->le_skin;
   h->k.le_y0 = 0.5 * (h->k.min_phys[1] + h->k.max_phys[1]);
+}
+
+// coordinates of the cells' lower faces (the FP32 offsets' origins)
+__global__ void k_axis_origins(Consts k, double* __restrict__ org) {
+  for (int a = 0; a < 3; ++a)
+    for (int c = threadIdx.x; c < k.nm[a]; c += blockDim.x)
+      org[a * k.org_pitch + c] = k.xmin[a] + (double)c * k.cs[a];
 }
 
 // conformation tensor: host (d*d, N) interleaved -> device [c][n]; identity
@@ -540,7 +563,7 @@ int ensure_capacity(Handle* h, int64_t n64) {
       // candidates within rc + skin: the list grows with the volume ratio
       const double rv = std::sqrt((double)h->k.rv2f) / h->p.cut_off;
       h->vcap = (int)std::ceil(neigh * std::pow(rv, d) * 1.05) + 8;
-      if ((rc = dalloc(h, &h->x_ref, cap)) ||
+      if ((rc = dalloc(h, &h->off_ref, cap)) ||
           (rc = dalloc(h, &h->vl, cap * (size_t)(8 * list_octets(h->vcap, two)))) ||
           (rc = dalloc(h, &h->vcount, cap)) || (rc = dalloc(h, &h->d_rebuild, 2)))
         return rc;
@@ -578,6 +601,12 @@ int ensure_capacity(Handle* h, int64_t n64) {
     if ((rc = dalloc(h, &h->up_x, cap * 9)) || (rc = dalloc(h, &h->up_v, cap * 3)) ||
         (rc = dalloc(h, &h->up_m, cap)) || (rc = dalloc(h, &h->up_id, cap * 2)))
       return rc;
+    h->k.org_pitch = std::max(h->k.nm[0], std::max(h->k.nm[1], h->k.nm[2]));
+    if ((rc = dalloc(h, &h->org, 3 * (size_t)h->k.org_pitch))) return rc;
+    h->k.org = h->org;
+    k_axis_origins<<<1, 256, 0, h->stream>>>(h->k, h->org);
+    h->launches++;
+    if (cuda_check(h, cudaGetLastError(), "cell origins")) return MCFG_ECUDA;
     h->up_cap = cap;
     h->cap_n = n;
     if (cuda_check(h, cudaMemsetAsync(h->d_err, 0, sizeof(unsigned), h->stream), "memset err"))
@@ -790,7 +819,8 @@ void boundary_update(Handle* h, double time_r, double time_v) {
     if (k.reuse && h->reuse_valid && m > 0.0) {
       k.le_dS = dS;
       k.le_aff = dS / k.len[1];
-      k.half_skin_le2 = m * m;
+      k.le_afff = (float)k.le_aff;
+      far_bound(k, m);
     } else {
       le_map(h);
       h->reuse_valid = false;
@@ -814,7 +844,8 @@ void le_map(Handle* h) {
   k.le_pl = q - cl;
   k.le_dS = 0.0;
   k.le_aff = 0.0;
-  k.half_skin_le2 = k.half_skin2;
+  k.le_afff = 0.0f;
+  far_bound(k, 0.5 * h->le_skin);
   h->le_S_ref = S;
 }
 

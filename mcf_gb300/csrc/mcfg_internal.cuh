@@ -55,6 +55,7 @@ struct Consts {
   // stencil of the rebuild still holds every pair of the step.
   int reuse;
   double half_skin2;        // (skin/2)^2
+  float far2f;              // FP32 bound on a squared displacement, see far_bound
   float rv2f;               // FP32 bound of the candidate list, (rc + skin)^2 with slack
   // kernel
   int kernel_type;
@@ -82,13 +83,13 @@ struct Consts {
   // that shift moves the images of their slot offsets (0 otherwise).  The
   // rebuild test then measures displacements against the shear the faces
   // impose: x - x_ref - le_aff (y_ref - le_y0), le_aff = le_dS / L_y,
-  // against a bound whose square is half_skin_le2.
+  // against far2f.
   int le, ns;
   double le_S, le_dv;
   int le_cu, le_cl;
   double le_pu, le_pl;
   double le_dS, le_aff, le_y0;
-  double half_skin_le2;
+  float le_afff;         // le_aff in FP32
   // physics
   int rhs_density_type, rhs_force_type, eos_type;
   double c2, rho_ref, gamma, p0;
@@ -102,6 +103,9 @@ struct Consts {
   // colloids (boundary particles sid = 1..ncoll)
   int ncoll, coll_noslip, coll_rho_type, coll_translate, coll_rotate, pp_cc;
   double coll_dout;
+  // coordinates of the cells' lower faces along each axis, [3][org_pitch]
+  const double* org;
+  int org_pitch;
   const double* coll;    // device [ncoll][12]: X(3) V(3) Omega(3) R pad(2)
   float* collf;          // the same in FP32, behind it (the FP32 pair terms read it:
                          // a conversion is an FP64 instruction a pair)
@@ -112,6 +116,7 @@ struct Consts {
   uint32_t rk[20];       // its round keys (key + r * Weyl increment), taken
                          // from the parameter bank by the unrolled rounds
   int body_force_type;
+  int body_on;           // bit a: |body_force[a]| > machine_zero
   double body_force[3];
   double machine_zero;
   float machine_zerof;
@@ -232,11 +237,12 @@ struct Handle {
   int* up_id = nullptr;
   size_t up_cap = 0;
   // ---- neighbour-list reuse ----
-  double4_32a* x_ref = nullptr;  // positions at the last rebuild
+  float4* off_ref = nullptr;     // cell offsets at the last rebuild (w = y - le_y0)
   uint16_t* vl = nullptr;        // candidates within rc + skin, laid out as nl
   bool partitioned = false;      // FP32 lists: fluid-fluid candidates, then the others
   int* vcount = nullptr;         // [n]
   int vcap = 0;
+  double* org = nullptr;         // [3][max nm] cell origins per axis
   int* d_rebuild = nullptr;      // [0] rebuild request, [1] rebuilds done
   bool reuse_valid = false;      // the candidate list matches the particle order
   bool unwrapped = false;        // positions may lie outside periodic faces (list reuse)
@@ -410,6 +416,13 @@ enum { kForceOnly = 0, kForceBody = 1, kForceBodyKick = 2 };
 // ------------------------------------------------------------------------
 // Device helpers
 // ------------------------------------------------------------------------
+
+// half of a positive number, exactly (a multiplication by 0.5 is an FP64
+// instruction; (0.5 f) dt and f (dt / 2) round alike)
+__device__ __forceinline__ double halved(double a) {
+  if (__double2hiint(a) < 0x00200000) return 0.5 * a;
+  return __hiloint2double(__double2hiint(a) - 0x00100000, __double2loint(a));
+}
 
 // Philox4x32-10, Salmon et al., SC'11 ("Parallel random numbers: as easy as
 // 1, 2, 3"): multipliers and Weyl key increments of the published algorithm.

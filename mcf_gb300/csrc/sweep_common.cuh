@@ -289,11 +289,11 @@ __device__ __forceinline__ void force_epilogue(const Consts& k, int i, int si, c
     // particles_apply_body_force.F90:96-353
     const double g[3] = {k.body_force[0], k.body_force[1], k.body_force[2]};
     if (k.body_force_type == 1) {
-      if (fabs(g[0]) > k.machine_zero) ax += g[0];
-      if (fabs(g[1]) > k.machine_zero) ay += g[1];
-      if (D == 3 && fabs(g[2]) > k.machine_zero) az += g[2];
+      if (k.body_on & 1) ax += g[0];
+      if (k.body_on & 2) ay += g[1];
+      if (D == 3 && (k.body_on & 4)) az += g[2];
     } else if (k.body_force_type == 2) {
-      if (fabs(g[0]) > k.machine_zero) {
+      if (k.body_on & 1) {
         const double half = k.max_phys[D - 1] * 0.5;
         double xl = xi[D - 1];
         // positions may sit past a periodic face between list rebuilds
@@ -307,7 +307,7 @@ __device__ __forceinline__ void force_epilogue(const Consts& k, int i, int si, c
           ax -= g[0];
       }
     } else if (k.body_force_type == 3) {
-      if (fabs(g[0]) > k.machine_zero) {
+      if (k.body_on & 1) {
         const double kw = 2.0 * kPi / (k.max_phys[1] - k.min_phys[1]);
         ax += g[0] * sin(kw * xi[1]);
       }
@@ -319,9 +319,10 @@ __device__ __forceinline__ void force_epilogue(const Consts& k, int i, int si, c
     double4_32a vv = v[i];
     if (si == 0) {
       // rounded like k_integrate and the CPU restatement: v + (0.5 a) dt, no FMA
-      vv.x = __dadd_rn(vv.x, __dmul_rn(__dmul_rn(0.5, ax), dt));
-      vv.y = __dadd_rn(vv.y, __dmul_rn(__dmul_rn(0.5, ay), dt));
-      if (D == 3) vv.z = __dadd_rn(vv.z, __dmul_rn(__dmul_rn(0.5, az), dt));
+      const double hdt = halved(dt);
+      vv.x = __dadd_rn(vv.x, __dmul_rn(ax, hdt));
+      vv.y = __dadd_rn(vv.y, __dmul_rn(ay, hdt));
+      if (D == 3) vv.z = __dadd_rn(vv.z, __dmul_rn(az, hdt));
     } else if (si < 0 && k.walls) {
       // end of the step: the face's shear velocity (moving walls)
       double vs[3] = {vv.x, vv.y, vv.z};

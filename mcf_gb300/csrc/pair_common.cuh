@@ -60,6 +60,48 @@ struct ListTail {
   }
 };
 
+// The same for four candidates w at a time of which the bits of `hits` are kept.
+// lut (shared, filled by fill_keep_lut) compacts them: per mask two byte
+// selections of the four and two masks of the kept ones.
+struct QuadTail {
+  unsigned long long rest = 0;  // the last count % 4 entries, zero above
+  int count = 0;
+  __device__ __forceinline__ void append(uint16_t* list, bool up, int octets, int n, int i,
+                                         uint2 w, unsigned hits, const uint4* lut) {
+    const uint4 s = lut[hits];
+    const unsigned long long c =
+        ((unsigned long long)(__byte_perm(w.x, w.y, s.y) & s.w) << 32) |
+        (__byte_perm(w.x, w.y, s.x) & s.z);
+    const int r = count & 3, more = __popc(hits);
+    const unsigned long long low = rest | (c << (16 * r));
+    if (r + more >= 4) {
+      ListTail::put(list, up, count >> 2, octets, n, i,
+                    make_uint2((unsigned)low, (unsigned)(low >> 32)));
+      rest = r == 0 ? 0ull : c >> (64 - 16 * r);
+    } else {
+      rest = low;
+    }
+    count += more;
+  }
+  __device__ __forceinline__ void finish(uint16_t* list, bool up, int octets, int n, int i) const {
+    if (count & 3)
+      ListTail::put(list, up, count >> 2, octets, n, i,
+                    make_uint2((unsigned)rest, (unsigned)(rest >> 32)));
+  }
+};
+// entry of the table for a mask of four: the kept 16-bit entries packed low
+__device__ __forceinline__ uint4 keep_entry(unsigned m) {
+  unsigned sel[2] = {0u, 0u}, mask[2] = {0u, 0u};
+  int c = 0;
+  for (unsigned u = 0; u < 4; ++u)
+    if ((m >> u) & 1u) {
+      sel[c >> 1] |= ((2 * u) | ((2 * u + 1) << 4)) << (8 * (c & 1));
+      mask[c >> 1] |= 0xffffu << (16 * (c & 1));
+      ++c;
+    }
+  return make_uint4(sel[0], sel[1], mask[0], mask[1]);
+}
+
 struct NbTable {
   int start[kMaxStencil];
   int count[kMaxStencil];

@@ -50,10 +50,11 @@ __device__ __forceinline__ F2 raw_w2(const Consts& k, F2 d) {
 // (packed.cuh).  One lane a particle appends the kept entries four a store;
 // several lanes (small systems, lane l octets l, l + S, ...) place theirs by a
 // prefix sum, in candidate order.  Bound: issue and the latency of the gathers.
-// 261,568 particles, 113 candidates each: 116 us against 148 us one candidate
-// and 2-byte list load at a time.
+// 261,568 particles, 113 candidates each: 99 us (80 registers and 6 blocks a SM
+// 116, 64 and 8 102; gathering a group ahead 112 or more) against 148 us one
+// candidate and 2-byte list load at a time.
 template <int D, int S>
-__global__ void __launch_bounds__(kReuseTPB)
+__global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 1)
     k_density_list(Consts k, const int* __restrict__ cell_start, const int* __restrict__ cell_of,
                    const float4* __restrict__ off, const double4_32a* __restrict__ x,
                    const double4_32a* __restrict__ v, const double* __restrict__ m,
@@ -64,10 +65,12 @@ __global__ void __launch_bounds__(kReuseTPB)
                    unsigned long long* __restrict__ pairs, NN nn, CollArgs ca) {
   __shared__ int s_start[kMaxStencil * kReuseTPB / S];
   __shared__ float4 s_slot[kSlotTable];
+  __shared__ uint4 s_keep[16];
   const int n = k.n, tid = threadIdx.x;
   const int gt = blockIdx.x * kReuseTPB + tid;
   const int i = gt / S, lane_s = gt % S;
   fill_slot_offsets<D>(k, s_slot);
+  if (S == 1 && tid >= kReuseTPB - 16) s_keep[tid - (kReuseTPB - 16)] = keep_entry(tid & 15);
   __syncthreads();
   int kff = 0, ko = 0, si = 0;
   int idle = 0;  // pairs within the cut-off that no force acts in
@@ -83,7 +86,7 @@ __global__ void __launch_bounds__(kReuseTPB)
     const float4* slot_tab = slot_table(k, s_slot, celli);
     const float4 oi = off[i];
     si = __float_as_int(oi.w);
-    acc_i = dyn_rho(k, si);
+    acc_i = dyn_rho(k, si);  // else the density is constant and the sum unused
     const bool mass = k.rhs_density_type == 1;
     const int vc = vcount[i];
     const int nff = vc & 0xffff, ntot = nff + (vc >> 16);
@@ -121,6 +124,7 @@ __global__ void __launch_bounds__(kReuseTPB)
           // past the segment's end: out of the support
           if (p + u >= m_) rx[u] = 1e6f;
         }
+        F2 w[2];
 #pragma unroll
         for (int u = 0; u < 4; u += 2) {
           const F2 x2 = pack2(rx[u], rx[u + 1]), y2 = pack2(ry[u], ry[u + 1]);
@@ -131,19 +135,22 @@ __global__ void __launch_bounds__(kReuseTPB)
           }
           float d2v[2];
           unpack2(d2, d2v[0], d2v[1]);
-          if (acc_i) {
-            F2 w = raw_w2(k, pack2(sqrtf(d2v[0]), sqrtf(d2v[1])));
-            if (mass) w = mul2(w, pack2((float)m[j[u]], (float)m[j[u + 1]]));
-            // Kahan sums of the two halves; a rejected candidate adds its W
-            // of zero
-            const F2 y = sub2(w, cmp);
-            const F2 t = add2(acc, y);
-            cmp = sub2(sub2(t, acc), y);
-            acc = t;
-          }
+          w[u / 2] = raw_w2(k, pack2(sqrtf(d2v[0]), sqrtf(d2v[1])));
 #pragma unroll
           for (int h = 0; h < 2; ++h)
             if (d2v[h] < k.rc2f) hits |= 1u << (u + h);
+        }
+        if (mass) {
+          w[0] = mul2(w[0], pack2((float)m[j[0]], (float)m[j[1]]));
+          w[1] = mul2(w[1], pack2((float)m[j[2]], (float)m[j[3]]));
+        }
+        // Kahan sums of the two halves; a rejected candidate adds its W of zero
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const F2 y = sub2(w[u], cmp);
+          const F2 t = add2(acc, y);
+          cmp = sub2(sub2(t, acc), y);
+          acc = t;
         }
         if (!up) {
           // two boundary particles: counted, not listed for the force
@@ -160,26 +167,21 @@ __global__ void __launch_bounds__(kReuseTPB)
       uint4 nx = make_uint4(0, 0, 0, 0);
       if (8 * lane_s < m_) nx = octet(lane_s);
       if (S == 1) {
-        ListTail out;
+        QuadTail out;
+        auto keep = [&](int p, unsigned wx, unsigned wy) {
+          const unsigned e[4] = {wx & 0xffffu, wx >> 16, wy & 0xffffu, wy >> 16};
+          const unsigned hits = four(p, e);
+          if (in_place && out.count == p && (hits == 15u || p + __popc(hits) == m_))
+            out.count += __popc(hits);  // nothing rejected so far: the list holds them
+          else
+            out.append(nl, up, noct, n, i, make_uint2(wx, wy), hits, s_keep);
+        };
 #pragma unroll 1
         for (int p0 = 0; p0 < m_; p0 += 8) {
-          uint4 q = nx;
+          const uint4 q = nx;
           if (p0 + 8 < m_) nx = octet((p0 >> 3) + 1);
-#pragma unroll 1
-          for (int p = p0; p < min(p0 + 8, m_); p += 4) {
-            const unsigned e[4] = {q.x & 0xffffu, q.x >> 16, q.y & 0xffffu, q.y >> 16};
-            q.x = q.z;
-            q.y = q.w;
-            const unsigned hits = four(p, e);
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if ((hits >> u) & 1u) {
-                out.push(e[u]);
-                // nothing rejected so far: the list in place holds it
-                if (out.full() && !(in_place && out.count == p + u + 1))
-                  out.store(nl, up, noct, n, i);
-              }
-          }
+          keep(p0, q.x, q.y);
+          if (p0 + 4 < m_) keep(p0 + 4, q.z, q.w);
         }
         if (!(in_place && out.count == m_)) out.finish(nl, up, noct, n, i);
         kept = out.count;

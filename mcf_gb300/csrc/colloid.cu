@@ -10,9 +10,9 @@
 // added, both accelerations recorded in their histories, the centres wrapped
 // back into the box, and every boundary particle is turned with its colloid
 // and put at the new centre.  Here that runs as three kernels per sub-step
-// with no host round trip: k_colloid_drag (update.cu, one warp per colloid),
+// with no host round trip: k_colloid_drag (update.cu, a block per colloid),
 // k_colloid_rigid (one block, a thread per colloid, the O(N_c) and O(N_c^2)
-// parts) and k_colloid_follow (a warp per colloid over its boundary
+// parts) and k_colloid_follow (a block per colloid over its boundary
 // particles, which also commits the colloid's new centre, velocity and
 // angular velocity to the table the pair sweeps read).  All arithmetic is
 // FP64 in the operation order of the Fortran (no fused multiply-add), so the
@@ -77,7 +77,7 @@ __device__ __forceinline__ double ab_incr(int order, const double* h, double dt)
       return __dmul_rn(h[0], dt);
     case 2:
       s = __dsub_rn(__dmul_rn(3.0, h[0]), h[3]);
-      return __ddiv_rn(__dmul_rn(s, dt), 2.0);
+      return __dmul_rn(__dmul_rn(s, dt), 0.5);  // exactly the quotient by 2
     case 3:
       s = __dsub_rn(__dmul_rn(23.0, h[0]), __dmul_rn(16.0, h[3]));
       s = __dadd_rn(s, __dmul_rn(5.0, h[6]));
@@ -199,8 +199,27 @@ __global__ void k_colloid_rigid(Consts k, RigidArgs a) {
     for (int q = 0; q < D; ++q) xc[q] = a.xnew[(size_t)c * 3 + q];
     double rep[3] = {0.0, 0.0, 0.0};
     if (a.repul_type >= 1) {
+      // most partners are out of reach: an FP32 distance with room for its
+      // rounding leaves them out (the exact test took ~36 FP64 instructions a
+      // partner, 64 cycles each)
+      float xf[3] = {0.f, 0.f, 0.f}, extent = 0.f;
+#pragma unroll
+      for (int q = 0; q < D; ++q) {
+        xf[q] = narrow(xc[q]);
+        extent = fmaxf(extent, fmaxf(fabsf(narrow(k.min_phys[q])), fabsf(narrow(k.max_phys[q]))));
+      }
+      const float reach0 = narrow(rad_c) + 5.0f * narrow(a.hn) + 1e-5f * extent;
       for (int j = 0; j < nc; ++j) {
         if (j == c) continue;
+        float near2 = 0.f;
+#pragma unroll
+        for (int q = 0; q < D; ++q) {
+          float t = fabsf(xf[q] - narrow(a.xnew[(size_t)j * 3 + q]));
+          if (k.periodic[q] && t > 0.5f * narrow(k.len[q])) t = t - narrow(k.len[q]);
+          near2 += t * t;
+        }
+        const float reach = reach0 + narrow(k.coll[(size_t)j * 12 + 9]);
+        if (near2 > 1.0001f * reach * reach) continue;
         double R12[3] = {0.0, 0.0, 0.0}, rr = 0.0;
 #pragma unroll
         for (int q = 0; q < D; ++q) {
@@ -296,19 +315,17 @@ __global__ void k_colloid_rigid(Consts k, RigidArgs a) {
 // of its colloid's old centre, turned by the sub-step's rotation matrix, put
 // at the new centre in the same periodic image as before (so list reuse sees
 // a small displacement); then lane 0 writes the colloid's new centre,
-// velocity and angular velocity into the table the sweeps read.  One warp per
-// colloid: the warp reads only its own colloid's table row.
+// velocity and angular velocity into the table the sweeps read.  One block per
+// colloid (as k_colloid_drag): it reads only its own colloid's table row.
 template <int D>
-__global__ void k_colloid_follow(Consts k, const int* __restrict__ cstart,
+__global__ void __launch_bounds__(kCollTPB) k_colloid_follow(Consts k, const int* __restrict__ cstart,
                                  const int* __restrict__ cmem, const int* __restrict__ slot_of,
                                  const double* __restrict__ rec, const double* __restrict__ xnew,
                                  int rotate, double4_32a* __restrict__ x) {
-  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (c >= k.ncoll) return;
+  const int c = blockIdx.x;
   double* cd = const_cast<double*>(k.coll) + (size_t)c * 12;
   const double* r = rec + (size_t)c * kCollRec;
-  for (int q = cstart[c] + lane; q < cstart[c + 1]; q += 32) {
+  for (int q = cstart[c] + threadIdx.x; q < cstart[c + 1]; q += kCollTPB) {
     const int s = slot_of[cmem[q]];
     const double4_32a xv = x[s];
     const double xs[3] = {xv.x, xv.y, xv.z};
@@ -335,8 +352,8 @@ __global__ void k_colloid_follow(Consts k, const int* __restrict__ cstart,
     }
     x[s] = make_double4_32a(xo[0], xo[1], D == 3 ? xo[2] : 0.0, 0.0);
   }
-  __syncwarp();
-  if (lane == 0) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       cd[i] = xnew[(size_t)c * 3 + i];
@@ -386,13 +403,11 @@ int launch_rigid(Handle* h, const RigidArgs& a) {
 
 int launch_follow(Handle* h) {
   const int nc = h->k.ncoll;
-  const int warps_per_block = 4;
-  const int g = (nc + warps_per_block - 1) / warps_per_block;
   if (h->k.d == 3)
-    k_colloid_follow<3><<<g, 32 * warps_per_block, 0, h->stream>>>(
+    k_colloid_follow<3><<<nc, kCollTPB, 0, h->stream>>>(
         h->k, h->coll_start, h->coll_mem, h->slot_of, h->crec, h->cxnew, h->cp.rotate, h->x);
   else
-    k_colloid_follow<2><<<g, 32 * warps_per_block, 0, h->stream>>>(
+    k_colloid_follow<2><<<nc, kCollTPB, 0, h->stream>>>(
         h->k, h->coll_start, h->coll_mem, h->slot_of, h->crec, h->cxnew, h->cp.rotate, h->x);
   h->launches++;
   return cuda_check(h, cudaGetLastError(), "colloid follow launch") ? MCFG_ECUDA : MCFG_OK;

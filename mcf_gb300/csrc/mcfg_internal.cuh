@@ -407,6 +407,8 @@ int colloid_section(Handle* h, int64_t step, double dt);
 int colloid_initial(Handle* h);
 int colloid_drag_launch(Handle* h);
 int colloid_sync_host(Handle* h);
+// threads per colloid of the sweeps over its boundary particles
+constexpr int kCollTPB = 128;
 // doubles per colloid of the device record of the dynamics (colloid.cu)
 constexpr int kCollRec = 96;
 

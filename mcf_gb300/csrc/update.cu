@@ -204,19 +204,21 @@ __global__ void k_stats_final(const double* __restrict__ part, int nparts, doubl
   out[q] = s;
 }
 
-// particles_collect_colloid_interaction.F90:93-136: one warp per colloid
-// sums m f and r x (m f) over its boundary particles in a fixed order.
+// particles_collect_colloid_interaction.F90:93-136: a block of kCollTPB threads
+// per colloid sums m f and r x (m f) over its boundary particles in a fixed
+// order.  Bound: latency (gathers through slot_of, then ~35 dependent FP64
+// instructions a particle), so a colloid's ~265 particles are spread over four
+// warps: 32 -> 13 us for 59 colloids.
 template <int D>
-__global__ void k_colloid_drag(Consts k, const int* __restrict__ cstart,
-                               const int* __restrict__ cmem, const int* __restrict__ slot_of,
-                               const double4_32a* __restrict__ x,
-                               const double4_32a* __restrict__ f, const double* __restrict__ m,
-                               double* __restrict__ out) {
-  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (c >= k.ncoll) return;
+__global__ void __launch_bounds__(kCollTPB)
+    k_colloid_drag(Consts k, const int* __restrict__ cstart, const int* __restrict__ cmem,
+                   const int* __restrict__ slot_of, const double4_32a* __restrict__ x,
+                   const double4_32a* __restrict__ f, const double* __restrict__ m,
+                   double* __restrict__ out) {
+  __shared__ double part[kCollTPB / 32][6];
+  const int c = blockIdx.x, lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int q = cstart[c] + lane; q < cstart[c + 1]; q += 32) {
+  for (int q = cstart[c] + threadIdx.x; q < cstart[c + 1]; q += kCollTPB) {
     const int s = slot_of[cmem[q]];
     const double4_32a fv = f[s], xv = x[s];
     const double mi = m[s];
@@ -236,7 +238,13 @@ __global__ void k_colloid_drag(Consts k, const int* __restrict__ cstart,
 #pragma unroll
     for (int a = 0; a < 6; ++a) acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], o);
   if (lane == 0)
-    for (int a = 0; a < 6; ++a) out[(size_t)c * 6 + a] = acc[a];
+    for (int a = 0; a < 6; ++a) part[wib][a] = acc[a];
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    double sum = part[0][threadIdx.x];
+    for (int w = 1; w < kCollTPB / 32; ++w) sum += part[w][threadIdx.x];
+    out[(size_t)c * 6 + threadIdx.x] = sum;
+  }
 }
 
 // Boundary particles follow their colloid (particles_compute_colloid_
@@ -304,13 +312,11 @@ int colloid_move(Handle* h, const double* d_xnew, const double* d_rot) {
 int colloid_drag_launch(Handle* h) {
   const int nc = h->k.ncoll, d = h->k.d;
   if (nc == 0) return MCFG_OK;
-  const int warps_per_block = 4;
-  const int g = (nc + warps_per_block - 1) / warps_per_block;
   if (d == 3)
-    k_colloid_drag<3><<<g, 32 * warps_per_block, 0, h->stream>>>(
+    k_colloid_drag<3><<<nc, kCollTPB, 0, h->stream>>>(
         h->k, h->coll_start, h->coll_mem, h->slot_of, h->x, h->f, h->m, h->coll_out);
   else
-    k_colloid_drag<2><<<g, 32 * warps_per_block, 0, h->stream>>>(
+    k_colloid_drag<2><<<nc, kCollTPB, 0, h->stream>>>(
         h->k, h->coll_start, h->coll_mem, h->slot_of, h->x, h->f, h->m, h->coll_out);
   h->launches++;
   return cuda_check(h, cudaGetLastError(), "colloid drag launch") ? MCFG_ECUDA : MCFG_OK;

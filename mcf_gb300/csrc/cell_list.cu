@@ -6,6 +6,7 @@
 // :308-531 (rank2d alike), called each step from technique_build_list
 // (mcf/src/technique_build_list.F90:94-109, marching_integrate_VV.F90:968).
 #include "mcfg_internal.cuh"
+#include "sph.cuh"
 
 namespace mcfg {
 
@@ -15,9 +16,10 @@ namespace mcfg {
 // corrections at the upper boundary.  No contraction is possible here.
 __device__ __forceinline__ int ppm_axis_cell(double xa, double xmin, double xmax,
                                              double rdx, int nm) {
-  int ia = (int)floor(__dmul_rn(__dsub_rn(xa, xmin), rdx));
-  if (xa >= xmax && ia < nm) ia = nm;       // outside above: ghost layer
-  if (xa < xmax && ia >= nm) ia = nm - 1;   // inside: last real cell
+  int ia = __double2int_rd(__dmul_rn(__dsub_rn(xa, xmin), rdx));
+  const bool inside = less64(xa, xmax);
+  if (!inside && ia < nm) ia = nm;       // outside above: ghost layer
+  if (inside && ia >= nm) ia = nm - 1;   // inside: last real cell
   return (ia >= 0 && ia < nm) ? ia : -1;
 }
 
@@ -104,6 +106,7 @@ __global__ void k_scan_partials(int* part, int nparts, const int* __restrict__ g
   }
 }
 
+// part: the tiles' exclusive sums, null when there is one tile only
 __global__ void k_scan_final(const int* __restrict__ in, int n, const int* __restrict__ part,
                              int* __restrict__ out, const int* __restrict__ gate) {
   if (gate && *gate == 0) return;
@@ -117,7 +120,7 @@ __global__ void k_scan_final(const int* __restrict__ in, int n, const int* __res
     s += vals[e];
   }
   int total;
-  int run = block_exclusive_scan(s, smem, total) + part[blockIdx.x];
+  int run = block_exclusive_scan(s, smem, total) + (part ? part[blockIdx.x] : 0);
 #pragma unroll
   for (int e = 0; e < kScanPer; ++e) {
     if (base + e < n) out[base + e] = run;
@@ -173,11 +176,18 @@ __global__ void k_cell_finalize(Consts k, const int* __restrict__ start,
       org[a] = k.org[a * k.org_pitch + ca];
     }
   }
-  for (int e = lane; e < cnt; e += 32) {
-    const int o = order[s0 + e];
-    const int hm = hidx_in[o];
+  for (int e0 = 0; e0 < cnt; e0 += 32) {
+    const int e = e0 + lane;
+    const int o = e < cnt ? order[s0 + e] : 0;
+    const int hm = e < cnt ? hidx_in[o] : 0x7fffffff;
+    // the rank among the bin's host indices, 32 of them at a time from the lanes
     int r = 0;
-    for (int q = 0; q < cnt; ++q) r += (hidx_in[order[s0 + q]] < hm) ? 1 : 0;
+    for (int b = 0; b < cnt; b += 32) {
+      const int other = b == e0 ? hm : b + lane < cnt ? hidx_in[order[s0 + b + lane]] : 0x7fffffff;
+      const int m = min(32, cnt - b);
+      for (int q = 0; q < m; ++q) r += __shfl_sync(0xffffffffu, other, q) < hm ? 1 : 0;
+    }
+    if (e >= cnt) continue;
     const int dst = s0 + r;
     const double4_32a xp = x_in[o];
     x_out[dst] = xp;
@@ -190,9 +200,9 @@ __global__ void k_cell_finalize(Consts k, const int* __restrict__ start,
     slot_of[hm] = dst;
     cell_of[dst] = warp;
     float4 of;
-    of.x = (float)(xp.x - org[0]);
-    of.y = (float)(xp.y - org[1]);
-    of.z = (D == 3) ? (float)(xp.z - org[2]) : 0.0f;
+    of.x = narrow(xp.x - org[0]);
+    of.y = narrow(xp.y - org[1]);
+    of.z = (D == 3) ? narrow(xp.z - org[2]) : 0.0f;
     of.w = __int_as_float(sid_in[o]);  // species id rides in the w lane
     off[dst] = of;
     if (ct_in != nullptr) {
@@ -206,8 +216,8 @@ __global__ void k_cell_finalize(Consts k, const int* __restrict__ start,
       // distances to the two faces of the wall axis, formed in FP64 and
       // rounded once (boundary_noslip_solid.F90:200-206 uses x - x_sur)
       const double xa = k.wall_axis == 0 ? xp.x : (k.wall_axis == 1 ? xp.y : xp.z);
-      wd[dst] = make_float2((float)(xa - k.min_phys[k.wall_axis]),
-                            (float)(xa - k.max_phys[k.wall_axis]));
+      wd[dst] = make_float2(narrow(xa - k.min_phys[k.wall_axis]),
+                            narrow(xa - k.max_phys[k.wall_axis]));
     }
   }
 }
@@ -279,10 +289,14 @@ static int cell_list_launches(Handle* h, const int* gate) {
     h->launches++;
   }
   const int ntiles = (nbins + kScanTile - 1) / kScanTile;
-  k_scan_tiles<<<ntiles, kScanThreads, 0, s>>>(h->cnt, nbins, h->scan_part, gate);
-  k_scan_partials<<<1, 1024, 0, s>>>(h->scan_part, ntiles, gate);
-  k_scan_final<<<ntiles, kScanThreads, 0, s>>>(h->cnt, nbins, h->scan_part, h->cell_start, gate);
-  h->launches += 3;
+  if (ntiles > 1) {
+    k_scan_tiles<<<ntiles, kScanThreads, 0, s>>>(h->cnt, nbins, h->scan_part, gate);
+    k_scan_partials<<<1, 1024, 0, s>>>(h->scan_part, ntiles, gate);
+    h->launches += 2;
+  }
+  k_scan_final<<<ntiles, kScanThreads, 0, s>>>(h->cnt, nbins, ntiles > 1 ? h->scan_part : nullptr,
+                                               h->cell_start, gate);
+  h->launches++;
   if (n > 0) {
     k_scatter<<<gb, tb, 0, s>>>(n, h->key, h->rank, h->cell_start, h->order, gate);
     const int warps_per_block = 8;

@@ -452,8 +452,13 @@ __global__ void k_update_state(Consts k, int n, const int* __restrict__ slot_of,
     for (int a = 0; a < d; ++a) {
       xs[a] = hx[(size_t)hi * d + a];
       if (k.periodic[a]) {
-        const double sh = rint((cur[a] - xs[a]) / k.len[a]);
-        if (sh != 0.0) xs[a] = xs[a] + sh * k.len[a];
+        // less than half a period apart (tested on the integer pipe): the same
+        // image; the division is for the others
+        const double gap = cur[a] - xs[a];
+        if (!less64(fabs(gap), halved(k.len[a]))) {
+          const double sh = rint(gap / k.len[a]);
+          if (sh != 0.0) xs[a] = xs[a] + sh * k.len[a];
+        }
       }
     }
     x[s] = make_double4_32a(xs[0], xs[1], xs[2], 0.0);
@@ -490,8 +495,10 @@ __global__ void k_download_pos(Consts k, int n, const int* __restrict__ hidx,
   const double4_32a v = x[i];
   double xs[3] = {v.x, v.y, v.z};
   for (int a = 0; a < k.d; ++a) {
-    if (xs[a] < k.min_phys[a] && k.bc_lo[a] == MCFG_BC_PERIODIC) xs[a] = __dadd_rn(xs[a], k.len[a]);
-    if (xs[a] >= k.max_phys[a] && k.bc_hi[a] == MCFG_BC_PERIODIC) xs[a] = __dsub_rn(xs[a], k.len[a]);
+    if (k.bc_lo[a] == MCFG_BC_PERIODIC && less64(xs[a], k.min_phys[a]))
+      xs[a] = __dadd_rn(xs[a], k.len[a]);
+    if (k.bc_hi[a] == MCFG_BC_PERIODIC && !less64(xs[a], k.max_phys[a]))
+      xs[a] = __dsub_rn(xs[a], k.len[a]);
   }
   double* o = out + (size_t)hidx[i] * k.d;
   for (int a = 0; a < k.d; ++a) o[a] = xs[a];

@@ -426,6 +426,16 @@ __device__ __forceinline__ double halved(double a) {
   return __hiloint2double(__double2hiint(a) - 0x00100000, __double2loint(a));
 }
 
+// a < b on the integer pipe (an FP64 comparison is an instruction of the narrow
+// pipe).  As the comparison but for NaN (past every number) and the two zeros
+// (-0 before +0); a caller's result must not depend on those.
+__device__ __forceinline__ bool less64(double a, double b) {
+  long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
+  ia ^= (ia >> 63) & 0x7fffffffffffffffll;
+  ib ^= (ib >> 63) & 0x7fffffffffffffffll;
+  return ia < ib;
+}
+
 // Philox4x32-10, Salmon et al., SC'11 ("Parallel random numbers: as easy as
 // 1, 2, 3"): multipliers and Weyl key increments of the published algorithm.
 // rk: the 10 round keys, rk[2r] = k0 + r * 0x9E3779B9, rk[2r+1] = k1 + r *

@@ -13,10 +13,11 @@ namespace mcfg {
 
 // Periodic wrap of one coordinate, particles_adjust_particles.F90:150-161,
 // 268-279: x < min -> x + length; then x >= max -> x - length.  Solid-wall
-// faces only clamp wall particles to the total domain.
+// faces only clamp wall particles to the total domain.  (-0 wraps to L and back
+// to 0, NaN stays NaN.)
 __device__ __forceinline__ void wrap_axis(const Consts& k, int a,
                                           int sid, double& x, double& v) {
-  if (x < k.min_phys[a]) {
+  if (less64(x, k.min_phys[a])) {
     if (k.bc_lo[a] == MCFG_BC_PERIODIC) {
       x = __dadd_rn(x, k.len[a]);
     } else if (k.bc_lo[a] == MCFG_BC_WALL_SOLID) {
@@ -26,7 +27,7 @@ __device__ __forceinline__ void wrap_axis(const Consts& k, int a,
       }
     }
   }
-  if (x >= k.max_phys[a]) {
+  if (!less64(x, k.max_phys[a])) {
     if (k.bc_hi[a] == MCFG_BC_PERIODIC) {
       x = __dsub_rn(x, k.len[a]);
     } else if (k.bc_hi[a] == MCFG_BC_WALL_SOLID) {

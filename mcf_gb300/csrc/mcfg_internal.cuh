@@ -250,11 +250,14 @@ struct Handle {
   // The step is launch-bound below ~50k particles (14 launches a step); run_vv
   // replays a captured pair of steps instead (two: the fused second kick
   // swaps v and v2, so two steps bring the buffers back).  The force sweeps
-  // of the captured steps read the Philox step from d_step, which a one-thread
-  // kernel advances after every step.  A graph is reused while the handle's
+  // of the captured steps read the Philox step from d_step, which the kernel
+  // that opens the step advances (a one-thread kernel after the step where the
+  // colloids read it earlier).  A graph is reused while the handle's
   // constants and buffers are those it captured (graph_gen, v).
   int64_t* d_step = nullptr;
   bool graph_capturing = false;
+  bool graph_advance = false;    // while capturing: the step's opening moves d_step
+  bool stats_cleared = false;    // while capturing: it has cleared d_stats, d_pairs
   bool graph_off = false;        // capture failed once: plain launches from then on
   uint64_t graph_gen = 1;        // bumped whenever constants or buffers change
   struct GraphSlot {
@@ -263,6 +266,7 @@ struct Handle {
     double dt = 0.0;
     const void* v = nullptr;
     int64_t launches = 0;
+    bool advance = false;  // the steps move d_step at their opening
   } graphs[2];
   // mcfg_step_vv_host with page-locked host arrays replays a captured step:
   // inputs over, the step (positions back on the copy stream), velocities

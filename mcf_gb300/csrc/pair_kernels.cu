@@ -1172,9 +1172,10 @@ int compute_density(Handle* h, bool with_pressure, bool reuse) {
   Consts& k = h->k;
   cudaStream_t s = h->stream;
   const int n = (int)h->n;
-  if (cuda_check(h, cudaMemsetAsync(h->d_stats, 0, sizeof(int) * 4, s), "memset stats"))
-    return MCFG_ECUDA;
-  if (cuda_check(h, cudaMemsetAsync(h->d_pairs, 0, sizeof(unsigned long long), s), "memset pairs"))
+  if (!h->stats_cleared &&
+      (cuda_check(h, cudaMemsetAsync(h->d_stats, 0, sizeof(int) * 4, s), "memset stats") ||
+       cuda_check(h, cudaMemsetAsync(h->d_pairs, 0, sizeof(unsigned long long), s),
+                  "memset pairs")))
     return MCFG_ECUDA;
   if (n == 0) return MCFG_OK;
   const bool fp64 = h->p.precision == MCFG_PRECISION_FP64;

@@ -165,12 +165,15 @@ __global__ void __launch_bounds__(kReuseTPB, 4)
   __shared__ float4 s_slot[kSlotTable];
   __shared__ uint4 s_ring[kRing * kReuseTPB];
   const int n = k.n, tid = threadIdx.x;
+  if (n == 0) return;
   fill_slot_offsets<D>(k, s_slot);
   __syncthreads();
   const int gt = blockIdx.x * kReuseTPB + tid;
-  const int i = gt / S, lane_s = gt % S;
-  if (i >= n) return;  // the S lanes of a particle leave together
-  const int nc = ncount[i];
+  const int lane_s = gt % S;
+  if (S == 1 && gt >= n) return;
+  // lanes past the last particle stay for the block's end, with an empty list
+  const int i = S == 1 ? gt : min(gt / S, n - 1);
+  const int nc = S == 1 || gt / S < n ? ncount[i] : 0;
   const int nff = nc & 0xffff, no = nc >> 16;
   // the lane's octets: n0 of the first segment, then those of the second
   const int n0 = max(0, (nff + 7) / 8 - lane_s + S - 1) / S;
@@ -345,16 +348,41 @@ __global__ void __launch_bounds__(kReuseTPB, 4)
   float hi[3], lo[3];
 #pragma unroll
   for (int a = 0; a < D; ++a) join_sums<S>(acc[a], cmp[a], gmask, hi[a], lo[a]);
-  if (lane_s != 0) return;
+  int fi = i, fsi = si;  // the particle this thread finishes
+  float im = ci.z;
+  if (S > 1) {
+    constexpr int P = kFinish<S>;
+    float* s_sum = reinterpret_cast<float*>(s_start);
+    __syncthreads();
+    if (lane_s == 0) {
+#pragma unroll
+      for (int a = 0; a < D; ++a) {
+        s_sum[(2 * a) * P + tid / S] = hi[a];
+        s_sum[(2 * a + 1) * P + tid / S] = lo[a];
+      }
+    }
+    __syncthreads();
+    fi = blockIdx.x * P + tid;
+    if (tid >= P || fi >= n) return;
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+      hi[a] = s_sum[(2 * a) * P + tid];
+      lo[a] = s_sum[(2 * a + 1) * P + tid];
+    }
+    fsi = __float_as_int(off[fi].w);
+    float4 vi_, c_;
+    load_vc(vf, fi, vi_, c_);
+    im = c_.z;
+  }
   double tot[3] = {0.0, 0.0, 0.0};
 #pragma unroll
   for (int a = 0; a < D; ++a) {
-    const float p = hi[a] * ci.z;
-    tot[a] = widen(p) + widen(fmaf(hi[a], ci.z, -p) + lo[a] * ci.z);
+    const float p = hi[a] * im;
+    tot[a] = widen(p) + widen(fmaf(hi[a], im, -p) + lo[a] * im);
   }
-  const double4_32a xi4 = x[i];
+  const double4_32a xi4 = x[fi];
   const double xi[3] = {xi4.x, xi4.y, xi4.z};
-  force_epilogue<D>(k, i, si, xi, tot[0], tot[1], D == 3 ? tot[2] : 0.0, fuse_mode, dt, v, f,
+  force_epilogue<D>(k, fi, fsi, xi, tot[0], tot[1], D == 3 ? tot[2] : 0.0, fuse_mode, dt, v, f,
                     v_out, err);
 }
 

@@ -252,25 +252,26 @@ __global__ void __launch_bounds__(kReuseTPB)
                     CollArgs ca) {
   constexpr int CENTER = (D == 3) ? 13 : 4;
   __shared__ int s_start[kMaxStencil * kReuseTPB];
-  __shared__ int s_shift[kMaxStencil * kReuseTPB];
+  __shared__ __align__(8) int s_shift[kMaxStencil * kReuseTPB];
   const int n = k.n, tid = threadIdx.x;
   const int gt = blockIdx.x * kReuseTPB + tid;
   const int i = gt / S, lane_s = gt % S;
   int my_max = 0;
   unsigned long long my_pairs = 0;
+  int si = 0, kept = 0, back = 0;  // back: kept entries before the forward half
+  bool acc_i = false;
+  double sum = 0.0;
   if (i < n) {
     const int celli = cell_of[i];
     build_lane_table<D, kReuseTPB>(k, celli, cell_start, s_start, s_shift);
     const int li = i - s_start[CENTER * kReuseTPB + tid];
-    const int si = sid[i];
-    const bool acc_i = dyn_rho(k, si);
+    si = sid[i];
+    acc_i = dyn_rho(k, si);
     const int cnt = vcount[i];
     const double4_32a xi4 = x[i];
     const double xi[3] = {xi4.x, xi4.y, xi4.z};
     const int gbase = (tid & 31) & ~(S - 1);
     const unsigned gmask = (S == 32 ? 0xffffffffu : (1u << S) - 1u) << gbase;
-    double sum = 0.0;
-    int kept = 0, back = 0;  // back: kept entries before the forward half
     for (int e0 = 0; e0 < cnt; e0 += S) {
       const int e = e0 + lane_s;
       bool in = false, fwd = false;
@@ -305,33 +306,50 @@ __global__ void __launch_bounds__(kReuseTPB)
         back += __popc(bf);
       }
     }
-    if (S > 1) {
-      const double part = sum;
-      sum = __shfl_sync(gmask, part, gbase);
-#pragma unroll
-      for (int q = 1; q < S; ++q) sum += __shfl_sync(gmask, part, gbase + q);
-    }
+  }
+  int fi = i;  // the particle this thread finishes
+  bool fin = i < n;
+  if (S > 1) {
+    double* s_sum = reinterpret_cast<double*>(s_shift);
+    __syncthreads();
+    s_sum[tid] = sum;
     if (lane_s == 0) {
-      if (kept > cap) atomicOr(err, kErrNeighOverflow);
-      my_max = kept;
-      kept = min(kept, cap);
-      ncount[i] = kept;
-      nhs[i] = min(back, kept);
-      my_pairs = (unsigned long long)kept;
-      const double mi = m[i];
-      double rho_out;
-      if (acc_i) {
-        rho_out = ((k.rhs_density_type == 1) ? k.w0 * mi : k.w0) + sum;
-      } else {
-        rho_out = (k.rhs_density_type == 1) ? k.init_density : k.init_density / mi;
-      }
-      rho[i] = rho_out;
-      if (!(rho_out > 0.0)) atomicOr(err, kErrZeroDensity);
-      if (with_pressure) {
-        const double4_32a vi4 =
-            (si > 0 && k.ncoll > 0) ? colloid_particle_update<D>(k, i, si, x[i], ca) : v[i];
-        write_particle_records<true>(k, i, rho_out, mi, pid[i], vi4, pr, pc, pcf, vf, nn);
-      }
+      s_start[tid / S] = kept;
+      s_start[kFinish<S> + tid / S] = back;
+    }
+    __syncthreads();
+    fi = blockIdx.x * kFinish<S> + tid;
+    fin = tid < kFinish<S> && fi < n;
+    if (fin) {
+      sum = s_sum[tid * S];
+#pragma unroll
+      for (int q = 1; q < S; ++q) sum += s_sum[tid * S + q];
+      kept = s_start[tid];
+      back = s_start[kFinish<S> + tid];
+      si = sid[fi];
+      acc_i = dyn_rho(k, si);
+    }
+  }
+  if (fin) {
+    if (kept > cap) atomicOr(err, kErrNeighOverflow);
+    my_max = kept;
+    kept = min(kept, cap);
+    ncount[fi] = kept;
+    nhs[fi] = min(back, kept);
+    my_pairs = (unsigned long long)kept;
+    const double mi = m[fi];
+    double rho_out;
+    if (acc_i) {
+      rho_out = ((k.rhs_density_type == 1) ? k.w0 * mi : k.w0) + sum;
+    } else {
+      rho_out = (k.rhs_density_type == 1) ? k.init_density : k.init_density / mi;
+    }
+    rho[fi] = rho_out;
+    if (!(rho_out > 0.0)) atomicOr(err, kErrZeroDensity);
+    if (with_pressure) {
+      const double4_32a vi4 =
+          (si > 0 && k.ncoll > 0) ? colloid_particle_update<D>(k, fi, si, x[fi], ca) : v[fi];
+      write_particle_records<true>(k, fi, rho_out, mi, pid[fi], vi4, pr, pc, pcf, vf, nn);
     }
   }
 #pragma unroll
@@ -366,15 +384,6 @@ __global__ void k_pressure(Consts k, const double* __restrict__ rho, const doubl
 // k_density_reuse; their sums are added in lane order.  9,216 2D Oldroyd-B particles (288 warps for 608
 // schedulers with one lane each): the adjoint of 20 steps 9.3 -> 7.6 ms.
 // ---------------------------------------------------------------------------
-template <int S>
-__device__ __forceinline__ double lane_sum(double part, unsigned gmask) {
-  const int base = (threadIdx.x & 31) & ~(S - 1);
-  double tot = __shfl_sync(gmask, part, base);
-#pragma unroll
-  for (int q = 1; q < S; ++q) tot += __shfl_sync(gmask, part, base + q);
-  return tot;
-}
-
 template <int D, bool NNW, int S>
 __global__ void __launch_bounds__(kReuseTPB)
     k_force64(Consts k, const int* __restrict__ cell_start, const int* __restrict__ cell_of,
@@ -391,13 +400,17 @@ __global__ void __launch_bounds__(kReuseTPB)
   // the Philox counter's step: the argument, or the device step counter
   // when the sweep runs inside a captured graph
   const uint32_t step = step_ptr ? (uint32_t)*step_ptr : step_arg;
-  __shared__ int s_start[kMaxStencil * kReuseTPB];
-  __shared__ int s_shift[kMaxStencil * kReuseTPB];
+  __shared__ __align__(8) int s_tab[2 * kMaxStencil * kReuseTPB];
+  int* const s_start = s_tab;
+  int* const s_shift = s_tab + kMaxStencil * kReuseTPB;
   const int n = k.n;
+  if (n == 0) return;
   const bool noise = k.noise != 0;
   const int gt = blockIdx.x * kReuseTPB + threadIdx.x;
-  const int i = gt / S, lane_s = gt % S;
-  if (i >= n) return;  // the S lanes of a particle leave together
+  const int lane_s = gt % S;
+  if (S == 1 && gt >= n) return;
+  // lanes past the last particle stay for the block's end, with an empty list
+  const int i = S == 1 ? gt : min(gt / S, n - 1);
   build_lane_table<D, kReuseTPB>(k, cell_of[i], cell_start, s_start, s_shift);
   const int si = sid[i];
   const int pidi = pid[i];
@@ -418,7 +431,7 @@ __global__ void __launch_bounds__(kReuseTPB)
   T sacc[9];
 #pragma unroll
   for (int a = 0; a < 9; ++a) sacc[a] = 0;
-  const int cnt = ncount[i];
+  const int cnt = S == 1 || gt / S < n ? ncount[i] : 0;
   for (int e = lane_s; e < cnt; e += S) {
     const int ent = nl[up_at(e, n, i)];
     const int sl = ent >> kLocalBits, q = ent & (kMaxCellCount - 1);
@@ -564,26 +577,51 @@ __global__ void __launch_bounds__(kReuseTPB)
         for (int a = 0; a < D; ++a) sacc[b * D + a] += r[a] * pa[b] * T(0.5);
     }
   }
+  int fi = i, fsi = si;  // the particle this thread finishes
+  double xf[3] = {xi[0], xi[1], xi[2]};
   if (S > 1) {
-    const unsigned gmask = group_mask<S>();
+    // planes of the block's partial sums: acc | L | stress
+    static_assert((D + 2 * D2) * 2 <= 2 * kMaxStencil, "partial sums fit over the tables");
+    double* s_sum = reinterpret_cast<double*>(s_tab);
+    const int tid = threadIdx.x;
+    __syncthreads();
 #pragma unroll
-    for (int a = 0; a < D; ++a) acc[a] = lane_sum<S>(acc[a], gmask);
-    if (nnw) {
+    for (int a = 0; a < D; ++a) s_sum[a * kReuseTPB + tid] = acc[a];
 #pragma unroll
-      for (int cc = 0; cc < D2; ++cc) L[cc] = lane_sum<S>(L[cc], gmask);
+    for (int cc = 0; cc < D2; ++cc) {
+      if (nnw) s_sum[(D + cc) * kReuseTPB + tid] = L[cc];
+      if (k.stress) s_sum[(D + D2 + cc) * kReuseTPB + tid] = sacc[cc];
     }
-    if (k.stress) {
+    __syncthreads();
+    fi = blockIdx.x * kFinish<S> + tid;
+    if (tid >= kFinish<S> || fi >= n) return;
+    // in lane order
+    auto total = [&](int c) {
+      const double* part = s_sum + c * kReuseTPB + tid * S;
+      double tot = part[0];
 #pragma unroll
-      for (int a = 0; a < D2; ++a) sacc[a] = lane_sum<S>(sacc[a], gmask);
+      for (int q = 1; q < S; ++q) tot += part[q];
+      return tot;
+    };
+#pragma unroll
+    for (int a = 0; a < D; ++a) acc[a] = total(a);
+#pragma unroll
+    for (int cc = 0; cc < D2; ++cc) {
+      if (nnw) L[cc] = total(D + cc);
+      if (k.stress) sacc[cc] = total(D + D2 + cc);
     }
-    if (lane_s != 0) return;
+    fsi = sid[fi];
+    const double4_32a xf4 = x[fi];
+    xf[0] = xf4.x;
+    xf[1] = xf4.y;
+    xf[2] = xf4.z;
   }
   if (k.stress) {
 #pragma unroll
-    for (int a = 0; a < D * D; ++a) st[(size_t)a * n + i] = sacc[a];
+    for (int a = 0; a < D * D; ++a) st[(size_t)a * n + fi] = sacc[a];
   }
-  if (nnw) nn_epilogue<D>(k, nn, i, L, fuse_mode, dt);
-  force_epilogue<D>(k, i, si, xi, acc[0], acc[1], D == 3 ? acc[2] : 0.0, fuse_mode, dt, v,
+  if (nnw) nn_epilogue<D>(k, nn, fi, L, fuse_mode, dt);
+  force_epilogue<D>(k, fi, fsi, xf, acc[0], acc[1], D == 3 ? acc[2] : 0.0, fuse_mode, dt, v,
                     f, v_out, err);
 }
 
@@ -594,7 +632,7 @@ __global__ void __launch_bounds__(kReuseTPB)
 // S lanes per particle (1, or 4 for small systems, where one thread per
 // particle leaves most of the GPU idle and each thread's serial pair loop
 // sets the time): lane l takes list entries l, l + S, ...; the lanes' sums
-// are added in lane order by the first lane, which runs the epilogue.
+// are added in lane order by the thread that runs its epilogue.
 // STRESS: the per-particle stress s_i += r_ij (x) a_ij / 2 is accumulated
 // (a compile-time switch: its nine sums would otherwise stay live across
 // the pair loop of every run).  The 3D Oldroyd-B instances take 4 blocks
@@ -618,14 +656,17 @@ __global__ void __launch_bounds__(kReuseTPB, (NNW && D == 3) ? 4 : 5)
   // tables keep every lane busy (2D cells hold ~9 particles)
   __shared__ int s_start[kMaxStencil * kReuseTPB];
   const int n = k.n;
+  if (n == 0) return;
   const bool noise = k.noise != 0;
   const bool walls = k.wall_axis != -1;
   __shared__ float4 s_slot[kSlotTable];
   fill_slot_offsets<D>(k, s_slot);
   __syncthreads();
   const int gt = blockIdx.x * kReuseTPB + threadIdx.x;
-  const int i = gt / S, lane_s = gt % S;
-  if (i >= n) return;  // the S lanes of a particle leave together
+  const int lane_s = gt % S;
+  if (S == 1 && gt >= n) return;
+  // lanes past the last particle stay for the block's end, with an empty list
+  const int i = S == 1 ? gt : min(gt / S, n - 1);
   const int celli = cell_of[i];
   build_lane_table<D, kReuseTPB, false>(k, celli, cell_start, s_start, nullptr);
   const float4* slot_tab = slot_table(k, s_slot, celli);
@@ -649,7 +690,7 @@ __global__ void __launch_bounds__(kReuseTPB, (NNW && D == 3) ? 4 : 5)
 #pragma unroll
   for (int a = 0; a < 9; ++a) sacc[a] = 0.f;
   // the list's two segments: fluid-fluid pairs, then the others
-  const int nc = ncount[i];
+  const int nc = S == 1 || gt / S < n ? ncount[i] : 0;
   const int nff = nc & 0xffff, cnt = nff + (nc >> 16);
   JData nxt;
   int ent_n1 = 0;
@@ -729,51 +770,53 @@ __global__ void __launch_bounds__(kReuseTPB, (NNW && D == 3) ? 4 : 5)
         for (int a = 0; a < D; ++a) sacc[b * D + a] += r[a] * pa[b] * 0.5f;
     }
   }
+  int fi = i, fsi = si;  // the particle this thread finishes
   if (S > 1) {
-    // the lanes' sums, added in lane order by lane 0 of the group
-    const unsigned gmask = ((1u << S) - 1u) << ((threadIdx.x & 31) & ~(S - 1));
-    const int base = (threadIdx.x & 31) & ~(S - 1);
-    T part[3];
+    // planes of the block's partial sums: acc | L | stress
+    static_assert(D + 2 * D2 <= kMaxStencil, "partial sums fit over the table");
+    float* s_sum = reinterpret_cast<float*>(s_start);
+    const int tid = threadIdx.x;
+    __syncthreads();
 #pragma unroll
-    for (int a = 0; a < 3; ++a) part[a] = acc[a] - comp[a];
+    for (int a = 0; a < D; ++a) s_sum[a * kReuseTPB + tid] = acc[a] - comp[a];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      T tot = part[a];
-      for (int q = 1; q < S; ++q) tot += __shfl_sync(gmask, part[a], base + q);
-      acc[a] = tot;
-      comp[a] = 0.f;
+    for (int cc = 0; cc < D2; ++cc) {
+      if (nnw) s_sum[(D + cc) * kReuseTPB + tid] = L[cc];
+      if (STRESS) s_sum[(D + D2 + cc) * kReuseTPB + tid] = sacc[cc];
     }
-    if (nnw) {
+    __syncthreads();
+    fi = blockIdx.x * kFinish<S> + tid;
+    if (tid >= kFinish<S> || fi >= n) return;
+    // in lane order
+    auto total = [&](int c) {
+      const float* part = s_sum + c * kReuseTPB + tid * S;
+      T tot = part[0];
 #pragma unroll
-      for (int cc = 0; cc < D2; ++cc) {
-        T tot = L[cc];
-        for (int q = 1; q < S; ++q) tot += __shfl_sync(gmask, L[cc], base + q);
-        L[cc] = tot;
-      }
-    }
-    if (STRESS) {
+      for (int q = 1; q < S; ++q) tot += part[q];
+      return tot;
+    };
 #pragma unroll
-      for (int a = 0; a < 9; ++a) {
-        T tot = sacc[a];
-        for (int q = 1; q < S; ++q) tot += __shfl_sync(gmask, sacc[a], base + q);
-        sacc[a] = tot;
-      }
+    for (int a = 0; a < D; ++a) acc[a] = total(a);
+#pragma unroll
+    for (int cc = 0; cc < D2; ++cc) {
+      if (nnw) L[cc] = total(D + cc);
+      if (STRESS) sacc[cc] = total(D + D2 + cc);
     }
-    if (lane_s != 0) return;
+    fsi = __float_as_int(off[fi].w);
   }
   if (STRESS) {
 #pragma unroll
-    for (int a = 0; a < D * D; ++a) st[(size_t)a * n + i] = (double)sacc[a];
+    for (int a = 0; a < D * D; ++a) st[(size_t)a * n + fi] = (double)sacc[a];
   }
-  const double4_32a xi4 = x[i];
+  const double4_32a xi4 = x[fi];
   const double xi[3] = {xi4.x, xi4.y, xi4.z};
   if (nnw) {
     double Ld[D2];
 #pragma unroll
     for (int cc = 0; cc < D2; ++cc) Ld[cc] = (double)L[cc];
-    nn_epilogue<D>(k, nn, i, Ld, fuse_mode, dt);
+    nn_epilogue<D>(k, nn, fi, Ld, fuse_mode, dt);
   }
-  force_epilogue<D>(k, i, si, xi, (double)acc[0], (double)acc[1],
+  force_epilogue<D>(k, fi, fsi, xi, (double)acc[0], (double)acc[1],
                     D == 3 ? (double)acc[2] : 0.0, fuse_mode, dt, v, f, v_out, err);
 }
 

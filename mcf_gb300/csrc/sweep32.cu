@@ -52,9 +52,11 @@ __device__ __forceinline__ F2 raw_w2(const Consts& k, F2 d) {
 // prefix sum, in candidate order.  Bound: issue and the latency of the gathers.
 // 261,568 particles, 113 candidates each: 99 us (80 registers and 6 blocks a SM
 // 116, 64 and 8 102; gathering a group ahead 112 or more) against 148 us one
-// candidate and 2-byte list load at a time.
+// candidate and 2-byte list load at a time.  Four lanes need 104 registers
+// unless held to 5 blocks a SM, whose grid then ends in a nearly empty wave (41k
+// particles 58 us; 48 us with 88 registers).
 template <int D, int S>
-__global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 1)
+__global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 5)
     k_density_list(Consts k, const int* __restrict__ cell_start, const int* __restrict__ cell_of,
                    const float4* __restrict__ off, const double4_32a* __restrict__ x,
                    const double4_32a* __restrict__ v, const double* __restrict__ m,
@@ -75,7 +77,7 @@ __global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 1)
   int kff = 0, ko = 0, si = 0;
   int idle = 0;  // pairs within the cut-off that no force acts in
   bool acc_i = false;
-  double rho_i = 0.0;  // the sum over pairs
+  float hi = 0.0f, lo = 0.0f;  // the sum over pairs and its remainder
   if (i < n) {
     const unsigned gmask = group_mask<S>();
     const int celli = cell_of[i];
@@ -219,9 +221,7 @@ __global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 1)
       else
         ko = kept;
     }
-    float hi, lo;
     join_sums<S>(acc, cmp, gmask, hi, lo);
-    rho_i = widen(k.coeff) * (widen(hi) + widen(lo));
     if (S > 1) {
 #pragma unroll
       for (int w = 1; w < S; w <<= 1) idle += __shfl_xor_sync(gmask, idle, w);
@@ -229,29 +229,56 @@ __global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 1)
   }
   int my_max = 0;
   unsigned long long my_pairs = 0;
-  if (i < n && lane_s == 0) {
+  int fi = i;  // the particle this thread finishes
+  bool fin = i < n;
+  if (S > 1) {
+    constexpr int P = kFinish<S>;
+    const int group = tid / S;
+    __syncthreads();
+    if (lane_s == 0) {
+      s_start[group] = __float_as_int(hi);
+      s_start[P + group] = __float_as_int(lo);
+      s_start[2 * P + group] = kff;
+      s_start[3 * P + group] = ko;
+      s_start[4 * P + group] = idle;
+    }
+    __syncthreads();
+    fi = blockIdx.x * P + tid;
+    fin = tid < P && fi < n;
+    if (fin) {
+      hi = __int_as_float(s_start[tid]);
+      lo = __int_as_float(s_start[P + tid]);
+      kff = s_start[2 * P + tid];
+      ko = s_start[3 * P + tid];
+      idle = s_start[4 * P + tid];
+      si = __float_as_int(off[fi].w);
+      acc_i = dyn_rho(k, si);
+    }
+  }
+  if (fin) {
+    const double rho_i = widen(k.coeff) * (widen(hi) + widen(lo));
     const int kept = kff + ko + idle;
     if (kept > cap) {
       atomicOr(err, kErrNeighOverflow);
       kff = min(kff, cap);
       ko = min(ko, cap - kff);
     }
-    ncount[i] = kff | (ko << 16);
+    ncount[fi] = kff | (ko << 16);
     my_max = kept;
     my_pairs = (unsigned long long)kept;
-    const double mi = m[i];
+    const double mi = m[fi];
     double rho_out;
     if (acc_i) {
       rho_out = ((k.rhs_density_type == 1) ? k.w0 * mi : k.w0) + rho_i;
     } else {
       rho_out = (k.rhs_density_type == 1) ? k.init_density : k.init_density / mi;
     }
-    rho[i] = rho_out;
+    rho[fi] = rho_out;
     if (!(rho_out > 0.0)) atomicOr(err, kErrZeroDensity);
     if (with_pressure) {
       const double4_32a vi4 =
-          (si > 0 && k.ncoll > 0) ? colloid_particle_update<D>(k, i, si, x[i], ca) : v[i];
-      write_particle_records<false>(k, i, rho_out, mi, pid[i], vi4, pr, nullptr, pcf, vf, nn);
+          (si > 0 && k.ncoll > 0) ? colloid_particle_update<D>(k, fi, si, x[fi], ca) : v[fi];
+      write_particle_records<false>(k, fi, rho_out, mi, pid[fi], vi4, pr, nullptr, pcf, vf, nn);
     }
   }
 #pragma unroll

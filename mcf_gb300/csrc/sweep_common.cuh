@@ -225,6 +225,15 @@ inline int lanes32(int64_t n, int dim) {
   return n < kLanes16Below ? 16 : n < kLanes4Below ? 4 : 1;
 }
 
+// How a sweep with S > 1 lanes per particle ends: the lanes leave their sums in
+// shared memory (over the finished cell tables) and the block's first kFinish<S>
+// threads run the epilogue, a particle each.  Run by one lane in S, its ~80 FP64
+// instructions (64 cycles of a scheduler each, however few lanes take part) cost
+// S times as much: 16,384 2D Oldroyd-B particles, four lanes, FP64 pipe 40% busy
+// with it, force 25.7 us; so 20.0 us, density 18.5 -> 15.2.
+template <int S>
+constexpr int kFinish = kReuseTPB / S;
+
 // FP32 offset of each stencil slot (the neighbour cell's origin minus the
 // home cell's, w = Lees-Edwards velocity jump), build_table's t.o, in a
 // block-shared table of kSlotTable entries: slot s of a home cell in

@@ -76,3 +76,35 @@ def test_walls_and_pair_count(side):
         pairs.append(g.info()["num_pairs"])
     # FP32 separations may take a pair at the cut-off the other way
     assert abs(pairs[0] - pairs[1]) <= 1e-6 * pairs[1] + 2
+
+
+@pytest.mark.parametrize("precision", [PRECISION_FP64, PRECISION_FP32_MIXED])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 575])
+def test_last_block_of_an_oldroyd_b_system(n, precision):
+    # several lanes per particle: the last block's idle lanes, the epilogues
+    # run by the block's first threads (velocity, conformation tensor, stress)
+    from oracle.oracle import Oracle
+    w = configs.c5_oldroyd_b_2d(n_side=24)
+    w.params.stress_tensor = 1
+    w.params.precision, w.params.Brownian, w.params.kt = precision, 0, 0.0
+    rng = np.random.default_rng(n)
+    w.x = w.x + rng.uniform(-0.2, 0.2, w.x.shape)
+    w.v = rng.normal(0, 1e-2, w.v.shape)
+    g, o = SDPD(w.params), Oracle(w.params)
+    for s in (g, o):
+        s.upload(w.x[:n], w.v[:n], w.m[:n], w.id[:n])
+        s.marching_init_force(0)
+    fp64 = precision == PRECISION_FP64
+    a, b = g.download("rho", "f", "s"), o.download("rho", "f", "s")
+    assert np.abs(a["rho"] / b["rho"] - 1.0).max() <= (1e-12 if fp64 else DENSITY)
+    bar = 1e-12 if fp64 else FORCE
+    scale = o.force_scale()[:, None]
+    assert (np.abs(a["f"] - b["f"]) <= bar * (scale + np.abs(b["f"]))).all()
+    # s_i sums r (x) a / 2 over pairs within the cut-off
+    assert np.abs(a["s"] - b["s"]).max() <= bar * w.params.cut_off * scale.max()
+    for s in (g, o):
+        s.marching_integrate_VV(1, w.dt)
+    a, b = g.download("v", "ct"), o.download("v", "ct")
+    assert np.abs(a["v"] - b["v"]).max() <= bar * (np.abs(b["v"]).max() + w.dt * scale.max())
+    dev = np.abs(b["ct"] - np.array([1.0, 0, 0, 1.0])).max()
+    assert np.abs(a["ct"] - b["ct"]).max() <= (1e-12 if fp64 else 1e-3 * dev + 1e-9)

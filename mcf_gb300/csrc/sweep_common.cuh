@@ -215,10 +215,10 @@ constexpr int64_t kSplitBelow = 50000;
 constexpr int64_t kSplit8Below = 12000;
 // Lanes per particle of the packed FP32 sweeps: a lane takes whole octets of a
 // list, and a 2D particle has about four octets of pairs, a 3D one fourteen or
-// more.  Measured, us a step (lanes 16 / 4 / 1): 3D rc = 3 dx 6k particles 66 /
-// 84 / 191, 18k 114 / 91 / 170, 41k 189 / 150 / 185, 71k 296 / 194 / 206, 91k 350 /
-// 222 / 187; 3D rc = 4 dx 8k 76 / 84 / 226, 33k 201 / 139 / 211, 91k 503 / 328 / 342;
-// 2D 10k 59 / 36 / 46, 23k 87 / 49 / 47, 63k 188 / 77 / 55.
+// more.  Measured, us a step (lanes 16 / 4 / 1): 3D rc = 3 dx 6k particles 60 /
+// 73 / 160, 18k 97 / 80 / 145, 41k 170 / 132 / 161, 71k 272 / 185 / 183, 91k 327 /
+// 203 / 168; 3D rc = 4 dx 8k 73 / 69 / 174, 33k 185 / 146 / 168, 91k 483 / 314 / 308;
+// 2D 10k 40 / 30 / 39, 23k 50 / 39 / 40, 63k 87 / 69 / 47.
 constexpr int64_t kLanes16Below = 12000, kLanes4Below = 75000, kLanes4Below2D = 20000;
 inline int lanes32(int64_t n, int dim) {
   if (dim == 2) return n < kLanes4Below2D ? 4 : 1;

@@ -15,7 +15,7 @@
 //   - the next two partners' records are gathered during the current pairs.
 // The fluid-fluid entries come first; entries with a boundary particle take
 // the same loop, their velocities and coefficients replaced before packing.
-// 261,568 particles, 113 pairs each: 227 us, 340 warp instructions two pairs,
+// 261,568 particles, 113 pairs each: 234 us, 340 warp instructions two pairs,
 // against 302 us and 265 a pair of the scalar sweep (k_force32).
 //
 // Reference: particles_compute_interaction.F90:609-900, rhs_force_ff_Newtonian_

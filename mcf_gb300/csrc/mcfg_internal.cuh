@@ -82,7 +82,7 @@ struct Consts {
   // last rebuild (le_cu .. le_pl computed from it) and le_dS = le_S minus
   // that shift moves the images of their slot offsets (0 otherwise).  The
   // rebuild test then measures displacements against the shear the faces
-  // impose: x - x_ref - le_aff (y_ref - le_y0), le_aff = le_dS / L_y,
+  // impose: x - x(rebuild) - le_aff (y(rebuild) - le_y0), le_aff = le_dS / L_y,
   // against far2f.
   int le, ns;
   double le_S, le_dv;
@@ -247,8 +247,9 @@ struct Handle {
   bool reuse_valid = false;      // the candidate list matches the particle order
   bool unwrapped = false;        // positions may lie outside periodic faces (list reuse)
   // ---- CUDA graph of two list-reuse VV steps (mcfg_run_vv) ----
-  // The step is launch-bound below ~50k particles (14 launches a step); run_vv
-  // replays a captured pair of steps instead (two: the fused second kick
+  // The step is launch-bound below ~50k particles (14 launches and two clears a
+  // step); run_vv replays a captured pair of steps instead, four kernels each
+  // when no rebuild is due (two: the fused second kick
   // swaps v and v2, so two steps bring the buffers back).  The force sweeps
   // of the captured steps read the Philox step from d_step, which the kernel
   // that opens the step advances (a one-thread kernel after the step where the

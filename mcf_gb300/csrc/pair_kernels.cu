@@ -5,8 +5,9 @@
 // Candidates (k_scan): one warp owns one cell and walks its particles in
 // chunks of 32 (lane = particle i) through the 27 (3D) or 9 (2D) neighbour
 // cells, an FP32 test on cell offsets; the hits go to a per-particle list of
-// 16-bit entries slot<<11 | local index (octets, see pair_common.cuh).  With list reuse the list holds the candidates within rc + skin and
-// outlives the step, otherwise it is made for this step.
+// 16-bit entries slot<<11 | local index (octets, see pair_common.cuh).  With
+// list reuse the list holds the candidates within rc + skin and outlives the
+// step, otherwise it is made for this step.
 //
 // Density (k_density_reuse here for FP64, k_density_list in sweep32.cu for
 // FP32-mixed): thread per particle (several lanes each on small systems) over
@@ -16,7 +17,8 @@
 // evaluates the equation of state and writes the per-particle pair
 // coefficients.
 //
-// Force (k_force32, k_force64): walks the step's list and gathers the pair
+// Force (k_force32_packed in force32.cu for the common FP32 forms, k_force32 for
+// the others, k_force64): walks the step's list and gathers the pair
 // accelerations of particle i.  Each pair is evaluated from both sides, so
 // there is no scatter, no atomic and the result is deterministic; the random
 // term is keyed by the unordered pid pair, so both sides draw the same dW.
@@ -626,7 +628,8 @@ __global__ void __launch_bounds__(kReuseTPB)
 }
 
 // ---------------------------------------------------------------------------
-// FP32-mixed force sweep: pair arithmetic in FP32 on cell offsets, Kahan
+// FP32-mixed force sweep of Oldroyd-B, the Morris and Espanol forms and runs with
+// the per-particle stress (the other forms: force32.cu): pair arithmetic in FP32 on cell offsets, Kahan
 // sums, the next pair's data loaded while the current one is computed.
 // ---------------------------------------------------------------------------
 // S lanes per particle (1, or 4 for small systems, where one thread per

@@ -58,7 +58,7 @@ __device__ __forceinline__ double4_32a colloid_particle_update(const Consts& k, 
 }
 
 // Per-particle prologue of the force sweep: pressure from the equation of
-// state and the pair coefficients (fused into k_density or run as
+// state and the pair coefficients (fused into the density sweeps or run as
 // k_pressure).  The FP32 path forms them in FP32.
 template <bool FP64>
 __device__ __forceinline__ void write_particle_records(const Consts& k, int i, double rho, double m,

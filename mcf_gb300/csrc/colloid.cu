@@ -42,6 +42,9 @@ namespace {
 constexpr int kRecM = 0, kRecMmi = 1, kRecTheta = 4, kRecDrag = 7, kRecTorque = 10,
               kRecRot = 13, kRecAcc = 22, kRecV = 31, kRecOm = 46, kRecF = 61, kRecAl = 76;
 constexpr int kMaxAB = 5;
+// largest block of k_colloid_rigid, ~140 registers a thread: more colloids
+// make more trips
+constexpr int kRigidTPB = 256;
 static_assert(kRecAl + 3 * kMaxAB <= kCollRec, "colloid record too small");
 
 struct RigidArgs {
@@ -132,7 +135,7 @@ __device__ __forceinline__ void rotation_matrix(const double* ax, double phi, do
 // mode 1, the initial accelerations of marching_marching.F90:995-1110: B at
 // the current centres, then the rotate acceleration.
 template <int D>
-__global__ void k_colloid_rigid(Consts k, RigidArgs a) {
+__global__ void __launch_bounds__(kRigidTPB) k_colloid_rigid(Consts k, RigidArgs a) {
   const int nc = k.ncoll;
   const int64_t step = a.step_ptr ? *a.step_ptr : a.step_arg;
   for (int c = threadIdx.x; c < nc; c += blockDim.x) {
@@ -392,7 +395,7 @@ RigidArgs rigid_args(Handle* h, int64_t step, int isub, int mode, double dts) {
 
 int launch_rigid(Handle* h, const RigidArgs& a) {
   const int nc = h->k.ncoll;
-  const int bs = nc >= 1024 ? 1024 : ((nc + 31) / 32) * 32;
+  const int bs = nc >= kRigidTPB ? kRigidTPB : ((nc + 31) / 32) * 32;
   if (h->k.d == 3)
     k_colloid_rigid<3><<<1, bs, 0, h->stream>>>(h->k, a);
   else

@@ -202,3 +202,16 @@ def test_move_colloids_refused_while_integrating_on_device(gpu_lib):
     g, _ = pair(w, cs, cd, m, mmi)
     with pytest.raises(MCFGError):
         g.move_colloids(cs.x, None, cs.v, cs.omega)
+
+
+def test_many_colloids(gpu_lib):
+    # more colloids than the rigid-body block has threads and than a chunk of
+    # partners holds, some within reach of one another
+    w, cs, cd, m, mmi = case(ab=2, nsub=2, n_side=40, n_colloid=600, radius=1.2)
+    assert len(cs.x) == 600
+    cs.params.cc_repul_cut_off = 0.3  # reach 1.5; the gaps are 1 and more
+    g, o = pair(w, cs, cd, m, mmi)
+    for s in range(1, 4):
+        g.colloid_integrate(s, 2e-3)
+        o.colloid_integrate(s, 2e-3)
+    states_close(g.colloid_state(), o.colloid_state(), 40.0)

@@ -45,6 +45,7 @@ constexpr int kMaxAB = 5;
 // largest block of k_colloid_rigid, ~140 registers a thread: more colloids
 // make more trips
 constexpr int kRigidTPB = 256;
+constexpr int kNearChunk = 64;  // partners tested a chunk, a bit each
 static_assert(kRecAl + 3 * kMaxAB <= kCollRec, "colloid record too small");
 
 struct RigidArgs {
@@ -194,7 +195,11 @@ __global__ void __launch_bounds__(kRigidTPB) k_colloid_rigid(Consts k, RigidArgs
     for (int q = 0; q < 3; ++q) a.xnew[(size_t)c * 3 + q] = xn[q];
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+  __shared__ float4 s_near[kNearChunk];
+  // (every thread makes every trip: the chunks' barriers)
+  for (int c0 = 0; c0 < nc; c0 += blockDim.x) {
+    const bool live = c0 + (int)threadIdx.x < nc;
+    const int c = live ? c0 + threadIdx.x : nc - 1;
     double* r = a.rec + (size_t)c * kCollRec;
     const double rad_c = k.coll[(size_t)c * 12 + 9];
     double xc[3] = {0.0, 0.0, 0.0};
@@ -204,57 +209,81 @@ __global__ void __launch_bounds__(kRigidTPB) k_colloid_rigid(Consts k, RigidArgs
     if (a.repul_type >= 1) {
       // most partners are out of reach: an FP32 distance with room for its
       // rounding leaves them out (the exact test took ~36 FP64 instructions a
-      // partner, 64 cycles each)
-      float xf[3] = {0.f, 0.f, 0.f}, extent = 0.f;
+      // partner, 64 cycles each).  Those in reach are noted a bit each and
+      // taken afterwards, in index order: a warp then runs the exact term as
+      // often as its busiest thread has partners, not once for every partner
+      // that any of its threads reaches.  59 colloids: 110 us with every
+      // partner tested exactly, 69 with FP32 tests from global memory, 43 so (records staged too)
+      float xf[3] = {0.f, 0.f, 0.f}, lf[3] = {0.f, 0.f, 0.f}, extent = 0.f;
 #pragma unroll
       for (int q = 0; q < D; ++q) {
         xf[q] = narrow(xc[q]);
+        lf[q] = k.periodic[q] ? narrow(k.len[q]) : INFINITY;
         extent = fmaxf(extent, fmaxf(fabsf(narrow(k.min_phys[q])), fabsf(narrow(k.max_phys[q]))));
       }
       const float reach0 = narrow(rad_c) + 5.0f * narrow(a.hn) + 1e-5f * extent;
-      for (int j = 0; j < nc; ++j) {
-        if (j == c) continue;
-        float near2 = 0.f;
-#pragma unroll
-        for (int q = 0; q < D; ++q) {
-          float t = fabsf(xf[q] - narrow(a.xnew[(size_t)j * 3 + q]));
-          if (k.periodic[q] && t > 0.5f * narrow(k.len[q])) t = t - narrow(k.len[q]);
-          near2 += t * t;
+      for (int j0 = 0; j0 < nc; j0 += kNearChunk) {
+        __syncthreads();
+        for (int b = threadIdx.x; b < kNearChunk && j0 + b < nc; b += blockDim.x) {
+          const double* xj = a.xnew + (size_t)(j0 + b) * 3;
+          s_near[b] = make_float4(narrow(xj[0]), narrow(xj[1]), D == 3 ? narrow(xj[2]) : 0.f,
+                                  narrow(k.coll[(size_t)(j0 + b) * 12 + 9]));
         }
-        const float reach = reach0 + narrow(k.coll[(size_t)j * 12 + 9]);
-        if (near2 > 1.0001f * reach * reach) continue;
-        double R12[3] = {0.0, 0.0, 0.0}, rr = 0.0;
+        __syncthreads();
+        unsigned long long near = 0;
+        const int jn = live ? min(kNearChunk, nc - j0) : 0;
+#pragma unroll 4
+        for (int b = 0; b < jn; ++b) {
+          const float4 o = s_near[b];
+          const float oq[3] = {o.x, o.y, o.z};
+          float near2 = 0.f;
 #pragma unroll
-        for (int q = 0; q < D; ++q) {
-          double t = __dsub_rn(xc[q], a.xnew[(size_t)j * 3 + q]);
-          if (k.periodic[q]) {
-            if (t > 0.5 * k.len[q])
-              t = __dsub_rn(t, k.len[q]);
-            else if (t < -0.5 * k.len[q])
-              t = __dadd_rn(t, k.len[q]);
+          for (int q = 0; q < D; ++q) {
+            float t = fabsf(xf[q] - oq[q]);
+            if (t > 0.5f * lf[q]) t = t - lf[q];
+            near2 += t * t;
           }
-          R12[q] = t;
-          rr = __dadd_rn(rr, __dmul_rn(t, t));
+          const float reach = reach0 + o.w;
+          // (not greater: what FP32 cannot order is left to the exact test)
+          if (j0 + b != c && !(near2 > 1.0001f * reach * reach)) near |= 1ull << b;
         }
-        const double rd = sqrt(rr);
-        double hgap = __dsub_rn(rd, __dadd_rn(rad_c, k.coll[(size_t)j * 12 + 9]));
-        if (!(hgap < 5.0 * a.hn)) continue;
-        double F = 0.0;
-        if (a.repul_type == 1) {  // Hookean
-          if (hgap < a.hn) {
+        while (near) {
+          const int j = j0 + __ffsll((long long)near) - 1;
+          near &= near - 1;
+          double R12[3] = {0.0, 0.0, 0.0}, rr = 0.0;
+#pragma unroll
+          for (int q = 0; q < D; ++q) {
+            double t = __dsub_rn(xc[q], a.xnew[(size_t)j * 3 + q]);
+            if (k.periodic[q]) {
+              if (t > 0.5 * k.len[q])
+                t = __dsub_rn(t, k.len[q]);
+              else if (t < -0.5 * k.len[q])
+                t = __dadd_rn(t, k.len[q]);
+            }
+            R12[q] = t;
+            rr = __dadd_rn(rr, __dmul_rn(t, t));
+          }
+          const double rd = sqrt(rr);
+          double hgap = __dsub_rn(rd, __dadd_rn(rad_c, k.coll[(size_t)j * 12 + 9]));
+          if (!(hgap < 5.0 * a.hn)) continue;
+          double F = 0.0;
+          if (a.repul_type == 1) {  // Hookean
+            if (hgap < a.hn) {
+              if (hgap < a.hm) hgap = a.hm;
+              F = __dsub_rn(a.F0, __ddiv_rn(__dmul_rn(a.F0, hgap), a.hn));
+            }
+          } else {  // DLVO
             if (hgap < a.hm) hgap = a.hm;
-            F = __dsub_rn(a.F0, __ddiv_rn(__dmul_rn(a.F0, hgap), a.hn));
+            const double e1 = exp(__ddiv_rn(-hgap, a.hn)), e5 = exp(-5.0);
+            F = __dsub_rn(__ddiv_rn(__dmul_rn(__ddiv_rn(a.F0, a.hn), e1), __dsub_rn(1.0, e1)),
+                          __ddiv_rn(__dmul_rn(__ddiv_rn(a.F0, a.hn), e5), __dsub_rn(1.0, e5)));
           }
-        } else {  // DLVO
-          if (hgap < a.hm) hgap = a.hm;
-          const double e1 = exp(__ddiv_rn(-hgap, a.hn)), e5 = exp(-5.0);
-          F = __dsub_rn(__ddiv_rn(__dmul_rn(__ddiv_rn(a.F0, a.hn), e1), __dsub_rn(1.0, e1)),
-                        __ddiv_rn(__dmul_rn(__ddiv_rn(a.F0, a.hn), e5), __dsub_rn(1.0, e5)));
-        }
 #pragma unroll
-        for (int q = 0; q < D; ++q) rep[q] = __dadd_rn(rep[q], __dmul_rn(F, __ddiv_rn(R12[q], rd)));
+          for (int q = 0; q < D; ++q) rep[q] = __dadd_rn(rep[q], __dmul_rn(F, __ddiv_rn(R12[q], rd)));
+        }
       }
     }
+    if (!live) continue;
     const double m = r[kRecM];
 #pragma unroll
     for (int q = 0; q < D; ++q) {

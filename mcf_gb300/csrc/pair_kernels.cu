@@ -383,8 +383,11 @@ __global__ void k_pressure(Consts k, const double* __restrict__ rho, const doubl
 // ---------------------------------------------------------------------------
 // FP64 force sweep: Oldroyd-B, stress, colloids, Lees-Edwards (k_force_sym has
 // the rest).  S lanes per particle take every S-th entry, as in
-// k_density_reuse; their sums are added in lane order.  9,216 2D Oldroyd-B particles (288 warps for 608
-// schedulers with one lane each): the adjoint of 20 steps 9.3 -> 7.6 ms.
+// k_density_reuse; their sums are added in lane order.  9,216 2D Oldroyd-B
+// particles (288 warps for 608 schedulers with one lane each): the adjoint of 20
+// steps 9.3 -> 7.6 ms.  The FP64 pipe bounds it, so the particle's own factor and
+// the stress's half follow the loop, and W'/d and the velocity's part of L are
+// formed once a pair (55 -> 51 us a launch there).
 // ---------------------------------------------------------------------------
 template <int D, bool NNW, int S>
 __global__ void __launch_bounds__(kReuseTPB)
@@ -547,28 +550,32 @@ __global__ void __launch_bounds__(kReuseTPB)
     for (int a = 0; a < D; ++a) vij[a] = vi[a] - vj[a];
     float z[6];
     if (noise) pair_draw<D>(k.rhs_force_type, k.rk, step, pidi, pid[j], z);
-    T pa[3], si_s, sj_s;
+    T pa[3];
     pair_force<T, D>(k, r, inv_d, vij, Ai, Bi, Aj, Bj, gw, noise, z, inv_sqdt, pa);
     if (nnw) {
       // polymer part of the pressure-tensor force,
       // rhs_force_ff_non_Newtonian_HuAdams.F90:95-110, and the velocity
       // gradient of pp_vgt_ip.inc
+      const T gwu = gw * inv_d;
 #pragma unroll
       for (int b = 0; b < D; ++b) {
         T s_ = 0;
 #pragma unroll
         for (int a = 0; a < D; ++a) s_ += (qie[1 + a + D * b] + qj[1 + a + D * b]) * r[a];
-        pa[b] += gw * inv_d * s_;
+        pa[b] += gwu * s_;
       }
-      const T fac = gw * qie[0] * inv_d;
+      const T fac = -gwu * qie[0];
 #pragma unroll
-      for (int b = 0; b < D; ++b)
+      for (int a = 0; a < D; ++a) {
+        const T w = vij[a] * fac;
 #pragma unroll
-        for (int a = 0; a < D; ++a) L[a + D * b] += (vj[a] - vi[a]) * r[b] * fac;
+        for (int b = 0; b < D; ++b) L[a + D * b] += w * r[b];
+      }
     }
-    pair_scales<T>(k.rhs_force_type, ci.z, cj.z, si_s, sj_s);
+    if (k.rhs_force_type == 1) {
 #pragma unroll
-    for (int a = 0; a < D; ++a) pa[a] *= si_s;
+      for (int a = 0; a < D; ++a) pa[a] *= cj.z;
+    }
 #pragma unroll
     for (int a = 0; a < D; ++a) acc[a] += pa[a];
     if (k.stress) {
@@ -576,8 +583,17 @@ __global__ void __launch_bounds__(kReuseTPB)
 #pragma unroll
       for (int b = 0; b < D; ++b)
 #pragma unroll
-        for (int a = 0; a < D; ++a) sacc[b * D + a] += r[a] * pa[b] * T(0.5);
+        for (int a = 0; a < D; ++a) sacc[b * D + a] += r[a] * pa[b];
     }
+  }
+  // the particle's own factor (all forms but Morris'), and the half of
+  // the stress
+  const T own = k.rhs_force_type == 1 ? T(1) : ci.z;
+#pragma unroll
+  for (int a = 0; a < D; ++a) acc[a] *= own;
+  if (k.stress) {
+#pragma unroll
+    for (int a = 0; a < D2; ++a) sacc[a] *= T(0.5) * own;
   }
   int fi = i, fsi = si;  // the particle this thread finishes
   double xf[3] = {xi[0], xi[1], xi[2]};

@@ -470,6 +470,9 @@ __global__ void __launch_bounds__(kAdjTPB)
     }
   }
   const double qi = 1.0 / ni, m4kt = -4.0 * kt;
+  const double cb = 0.70710678118654752440;
+  const double cr = 0.81649658092772603273 / cb - 1.0;  // ca/cb - 1 (3D; none in 2D)
+  const double k_z = inv_sqdt * cb, k_df = 0.5 * m4kt * k_z;
   double lim[3] = {0, 0, 0};  // lam_i / m_i
 #pragma unroll
   for (int a = 0; a < D; ++a) lim[a] = d4(li4, a) * pci.z;
@@ -506,10 +509,9 @@ __global__ void __launch_bounds__(kAdjTPB)
     // random term f_r We, We = s (ca (e.z) e + cb (z - (e.z) e)), replayed from
     // the pair's keys exactly as pair_force draws it (s goes into z);
     // f_r = sqrt(-4 kT f_d)/sqrt(dt) and df_r/df_d = f_r/(2 f_d) =
-    // -2 kT/sqrt(dt) / sqrt(-4 kT f_d), from one reciprocal square root
-    const double cbn = 0.70710678118654752440;
-    const double cdn = 0.81649658092772603273 - cbn;  // ca - cb (3D; none in 2D)
-    double gz[3] = {0, 0, 0}, f_r = 0.0, dfr = 0.0, eg = 0.0;
+    // -2 kT/sqrt(dt) / sqrt(-4 kT f_d), from one root; c_z = f_r cb, dfz the same
+    // of df_r/df_d
+    double gz[3] = {0, 0, 0}, c_z = 0.0, dfz = 0.0, eg = 0.0;
     // f_d < 0, by its bits
     if (noise && (unsigned long long)__double_as_longlong(f_d) > 0x8000000000000000ull) {
       float z[6];
@@ -517,18 +519,18 @@ __global__ void __launch_bounds__(kAdjTPB)
       const float sg = z[5] < 0.0f ? -1.0f : 1.0f;
 #pragma unroll
       for (int a = 0; a < D; ++a) gz[a] = widen(sg * z[a]);
-      const double rs = rsqrt(m4kt * f_d);
-      f_r = m4kt * f_d * rs * inv_sqdt;
-      dfr = 0.5 * m4kt * rs * inv_sqdt;
+      double rs;
+      const double root = root64<true>(m4kt * f_d, rs);
+      c_z = root * k_z;
+      dfz = rs * k_df;
       if (D == 3) {
 #pragma unroll
         for (int a = 0; a < D; ++a) eg += ev[a] * gz[a];
       }
     }
     // the pair value's part along e (also the e part of its own derivative)
-    const double c_e = f_r * cdn;
+    const double c_e = c_z * cr;
     const double along = (D == 3) ? c_e * eg - f_c : -f_c;
-    const double c_z = f_r * cbn;
     // forward pair value g and its seed gbar = lam_i/m_i - lam_j/m_j + h w~ r
     const double hm = pci.z + pcj.z;
     double P[D2], Pr[3];
@@ -557,18 +559,16 @@ __global__ void __launch_bounds__(kAdjTPB)
       gbe += gb[a] * ev[a];
       gbz += gb[a] * gz[a];
     }
-    double gbWe = cbn * gbz;
-    if (D == 3) gbWe += cdn * eg * gbe;
-    const double fdb = gbv + gbWe * dfr;
+    const double gbW = (D == 3) ? gbz + cr * eg * gbe : gbz;
+    const double fdb = gbv + gbW * dfz;
     // X: what W' u multiplies in the pair's scalar
     double X = fdb * (eta * SB);
-    double rb[3];
 #pragma unroll
     for (int a = 0; a < D; ++a) {
       double s1 = 0.0;
 #pragma unroll
       for (int b = 0; b < D; ++b) s1 += wt[b * D + a] * g[b];
-      rb[a] = hm * s1;
+      xb[a] += hm * s1;
     }
     if (NNW) {
       // L term: W' u sum_ab Phi_ab (v_j - v_i)_a r_b
@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(kAdjTPB)
         }
         X += gb[b] * Pr[b] - s * r[b];
         phi_i += si * r[b];
-        rb[b] += gwu * (s3 - s);
+        xb[b] += gwu * (s3 - s);
         vb[b] -= gwu * sv;  // d/dv_i of (v_j - v_i)
         const double gr = gwu * gb[b];
 #pragma unroll
@@ -603,7 +603,6 @@ __global__ void __launch_bounds__(kAdjTPB)
     const double ug = u * along, uz = u * t;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
-      xb[a] += rb[a];
       xb[a] += ug * gb[a];
       if (D == 3) xb[a] += uz * gz[a];
       xb[a] += radial * ev[a];
@@ -611,10 +610,11 @@ __global__ void __launch_bounds__(kAdjTPB)
     }
     Bbar += fdb * gwu;
     Abar -= gbe * gw;
-    etab += fdb * SBg;
   }
+  // d/d eta: sum over pairs of fdb SB W' u, each pair's halves B_i and B_j left to
+  // its two particles
+  etab = Bbar * pci.y;
   Bbar *= eta;
-  etab *= 0.5;
   nbL *= qi;  // Lbi holds Lbar_i / n_i already
   for (int o = 1; o < split; o <<= 1) {
 #pragma unroll

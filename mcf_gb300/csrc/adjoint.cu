@@ -425,7 +425,9 @@ __global__ void k_adj_pre(Consts k, Tape tp, double phi, const double4_32a* __re
 // sum X, the noise's sign in its normals, per-particle factors after the loop,
 // the polymer's only with NNW, the e part of the noise only in 3D (ca = cb in
 // 2D).  Against each term by itself: 1M particles in 3D, 20 steps, whole gradient
-// 1582 -> 1438 ms; 9,216 2D Oldroyd-B particles, 20 steps 7254 -> 6890 us.
+// 1582 -> 1438 ms; 9,216 2D Oldroyd-B particles, 20 steps 7254 -> 6890 us; the noise
+// from one root and eta's partial after the loop 1389 -> 1383 ms, 6777 -> 6705 us.
+// 3D held to 128 registers for 4 blocks a SM: 1407 ms (spills).
 template <int D, bool NNW>
 __global__ void __launch_bounds__(kAdjTPB)
     k_adj_force(Consts k, Tape tp, const double4_32a* __restrict__ lam,

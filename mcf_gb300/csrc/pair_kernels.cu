@@ -1115,7 +1115,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     }
     constexpr int kHop = sym_warp_bytes<D, COOP>() / 8;
     const double* part0 = COOP ? reinterpret_cast<const double*>(smem_raw) : part;
-    __syncwarp();
+    // a shared cell's warps read each other's sums below: those of a cell without
+    // particles, which has met no barrier above, are its zeros
+    if (COOP)
+      __syncthreads();
+    else
+      __syncwarp();
     for (int s = COOP ? wib : 0; s < NSF; s += COOP ? kWarpsPerBlock : 1) {
       const int cs_ = t.count[CENTER + s], st_ = t.start[CENTER + s];
       if (cs_ > CC) continue;

@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(kReuseTPB, 4)
     if (__float_as_int(oi.x) == 0x7fabcdef) break;
     // a lone last pair: its twin is put out of the support, where every term
     // is an exact zero
-    if (!both) hb.r[0] = 1e6f;
+    if (!both) hb.r[0] = k.beyondf;
     F2 r[3], vij[3];
 #pragma unroll
     for (int a = 0; a < D; ++a) {

@@ -64,7 +64,6 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
            int* __restrict__ stats) {
   if (gate && *gate == 0) return;
   constexpr int CENTER = (D == 3) ? 13 : 4;
-  constexpr float kFar = 3e18f;  // padding: far from everything, its square finite
   __shared__ NbTable tab[kWarpsPerBlock];
   __shared__ __align__(16) float sb[kWarpsPerBlock][2][3][32];
   __shared__ unsigned s_mask[kWarpsPerBlock][kMaskRows][32];
@@ -95,7 +94,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
         b2 = 0;
         if (++sl < ns) jn = min(t.count[sl], kMaxCellCount);
       }
-      const float4 pad = make_float4(kFar, kFar, kFar, 0.f);
+      const float4 pad = make_float4(0.f, 0.f, 0.f, 0.f);
       float4 nx = (sl < ns && b2 + lane < jn) ? off[t.start[sl] + b2 + lane] : pad;
       while (sl < ns) {
         const int sl_c = sl, b_c = b2, mm = min(32, jn - b2);
@@ -148,8 +147,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
           mask = __funnelshift_l(__float_as_uint(d2), mask, 1);
           mask = __funnelshift_l(__float_as_uint(d3), mask, 1);
         }
-        // candidate c of the chunk at bit 31 - c
+        // candidate c of the chunk at bit 31 - c, the padding's bits cut off
         mask <<= 32 - q;
+        mask &= 0xffffffffu << (32 - mm);
         if (sl_c == CENTER) {
           const int self = i - t.start[CENTER] - b_c;
           if (self >= 0 && self < 32) mask &= ~(0x80000000u >> self);

@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 5)
           ry[u] = (oi.y - o[u].y) - so.y;
           if (D == 3) rz[u] = (oi.z - o[u].z) - so.z;
           // past the segment's end: out of the support
-          if (p + u >= m_) rx[u] = 1e6f;
+          if (p + u >= m_) rx[u] = k.beyondf;
         }
         F2 w[2];
 #pragma unroll

@@ -143,8 +143,11 @@ __global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 5)
             if (d2v[h] < k.rc2f) hits |= 1u << (u + h);
         }
         if (mass) {
-          w[0] = mul2(w[0], pack2((float)m[j[0]], (float)m[j[1]]));
-          w[1] = mul2(w[1], pack2((float)m[j[2]], (float)m[j[3]]));
+          // W before the mass: a term is of the density's own size, whatever the
+          // units of mass and length (below 1.2e-38 it would be flushed to zero)
+          const F2 cw = splat2(k.coeff);
+          w[0] = mul2(mul2(cw, w[0]), pack2((float)m[j[0]], (float)m[j[1]]));
+          w[1] = mul2(mul2(cw, w[1]), pack2((float)m[j[2]], (float)m[j[3]]));
         }
         // Kahan sums of the two halves; a rejected candidate adds its W of zero
 #pragma unroll
@@ -256,7 +259,8 @@ __global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 5)
     }
   }
   if (fin) {
-    const double rho_i = widen(k.coeff) * (widen(hi) + widen(lo));
+    const double sum = widen(hi) + widen(lo);
+    const double rho_i = k.rhs_density_type == 1 ? sum : widen(k.coeff) * sum;
     const int kept = kff + ko + idle;
     if (kept > cap) {
       atomicOr(err, kErrNeighOverflow);

@@ -231,7 +231,7 @@ __global__ void k_zero_counts(int* __restrict__ cnt, int nbins, const int* __res
 
 // after a gated rebuild: the permuted state back into the primary buffers
 // (a host-side pointer swap cannot depend on the device flag) and the
-// reference offsets of the new candidate list
+// reference positions and offsets of the new candidate list
 template <int D>
 __global__ void k_copy_back(int n, const int* __restrict__ gate, const double4_32a* __restrict__ x2,
                             const double4_32a* __restrict__ v2, const double4_32a* __restrict__ f2,
@@ -243,12 +243,13 @@ __global__ void k_copy_back(int n, const int* __restrict__ gate, const double4_3
                             int* __restrict__ pid, int* __restrict__ sid, int* __restrict__ hidx,
                             double* __restrict__ ct, double* __restrict__ act,
                             const float4* __restrict__ off, double y0,
-                            float4* __restrict__ off_ref) {
+                            double4_32a* __restrict__ x_ref, float4* __restrict__ off_ref) {
   if (*gate == 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double4_32a xp = x2[i];
   x[i] = xp;
+  x_ref[i] = xp;
   const float4 of = off[i];
   off_ref[i] = make_float4(of.x, of.y, of.z, (float)(xp.y - y0));
   v[i] = v2[i];
@@ -328,7 +329,8 @@ static int cell_list_launches(Handle* h, const int* gate) {
 #define COPY_BACK(DD)                                                                            \
   k_copy_back<DD><<<gb, tb, 0, s>>>(n, gate, h->x2, h->v2, h->f2, h->m2, h->pid2, h->sid2,       \
                                     h->hidx2, h->ct2, h->act2, h->x, h->v, h->f, h->m, h->pid,   \
-                                    h->sid, h->hidx, h->ct, h->act, h->off, k.le_y0, h->off_ref)
+                                    h->sid, h->hidx, h->ct, h->act, h->off, k.le_y0, h->x_ref,    \
+                                    h->off_ref)
       if (k.d == 3) COPY_BACK(3); else COPY_BACK(2);
 #undef COPY_BACK
       h->launches++;

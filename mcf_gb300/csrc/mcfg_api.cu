@@ -145,8 +145,9 @@ void free_all(Handle* h) {
   h->out_dev = nullptr;
   h->out_host = nullptr;
   h->out_cap = 0;
-  for (void* p : {(void*)h->off_ref, (void*)h->org, (void*)h->vl, (void*)h->vcount, (void*)h->d_rebuild})
+  for (void* p : {(void*)h->x_ref, (void*)h->off_ref, (void*)h->org, (void*)h->vl, (void*)h->vcount, (void*)h->d_rebuild})
     if (p) cudaFree(p);
+  h->x_ref = nullptr;
   h->off_ref = nullptr;
   h->org = nullptr;
   h->k.org = nullptr;
@@ -250,14 +251,18 @@ namespace {
 
 namespace mcfg {
 
-// The rebuild test runs in FP32 on cell offsets: each is rounded (6e-8 of a
-// cell side), so the bound on their difference is drawn in by more than two
-// such roundings an axis can make (and, sheared, by that of y_ref le_aff).
+// The rebuild test asks in FP64 whether a particle has moved more than half.
+// FP32 cell offsets answer it but for displacements nearer to half than
+// their own roundings (6e-8 of a cell side each) can shift them, two an axis
+// (and, sheared, that of y_ref le_aff).
 void far_bound(Consts& k, double half) {
   double side = 0.0;
   for (int a = 0; a < k.d; ++a) side = std::max(side, k.cs[a]);
-  const double b = std::max(0.0, half - 4e-7 * side - 2e-7 * std::fabs(k.le_aff) * k.len[1]);
-  k.far2f = (float)(b * b * (1.0 - 1e-6));
+  const double room = 4e-7 * side + 2e-7 * std::fabs(k.le_aff) * k.len[1];
+  const double lo = half - room, hi = half + room;
+  k.far2 = half * half;
+  k.near2f = lo > 0.0 ? (float)(lo * lo * (1.0 - 1e-6)) : -1.0f;
+  k.far2f = (float)(hi * hi * (1.0 + 1e-6));
 }
 
 void make_consts(const mcfg_params& p, Consts& k) {
@@ -571,7 +576,7 @@ int ensure_capacity(Handle* h, int64_t n64) {
       // candidates within rc + skin: the list grows with the volume ratio
       const double rv = std::sqrt((double)h->k.rv2f) / h->p.cut_off;
       h->vcap = (int)std::ceil(neigh * std::pow(rv, d) * 1.05) + 8;
-      if ((rc = dalloc(h, &h->off_ref, cap)) ||
+      if ((rc = dalloc(h, &h->x_ref, cap)) || (rc = dalloc(h, &h->off_ref, cap)) ||
           (rc = dalloc(h, &h->vl, cap * (size_t)(8 * list_octets(h->vcap, two)))) ||
           (rc = dalloc(h, &h->vcount, cap)) || (rc = dalloc(h, &h->d_rebuild, 2)))
         return rc;
@@ -867,6 +872,7 @@ void le_map(Handle* h) {
   k.le_aff = 0.0;
   k.le_afff = 0.0f;
   far_bound(k, 0.5 * h->le_skin);
+  k.far2 = k.half_skin2;
   h->le_S_ref = S;
 }
 

@@ -57,7 +57,10 @@ struct Consts {
   // stencil of the rebuild still holds every pair of the step.
   int reuse;
   double half_skin2;        // (skin/2)^2
-  float far2f;              // FP32 bound on a squared displacement, see far_bound
+  // bound on a squared displacement since the last rebuild, and the two FP32
+  // bounds below and above which FP32 offsets decide alike (far_bound)
+  double far2;
+  float near2f, far2f;
   float rv2f;               // FP32 bound of the candidate list, (rc + skin)^2 with slack
   // kernel
   int kernel_type;
@@ -85,7 +88,7 @@ struct Consts {
   // that shift moves the images of their slot offsets (0 otherwise).  The
   // rebuild test then measures displacements against the shear the faces
   // impose: x - x(rebuild) - le_aff (y(rebuild) - le_y0), le_aff = le_dS / L_y,
-  // against far2f.
+  // against far2.
   int le, ns;
   double le_S, le_dv;
   int le_cu, le_cl;
@@ -239,7 +242,8 @@ struct Handle {
   int* up_id = nullptr;
   size_t up_cap = 0;
   // ---- neighbour-list reuse ----
-  float4* off_ref = nullptr;     // cell offsets at the last rebuild (w = y - le_y0)
+  double4_32a* x_ref = nullptr;  // positions at the last rebuild
+  float4* off_ref = nullptr;     // cell offsets then (w = y - le_y0)
   uint16_t* vl = nullptr;        // candidates within rc + skin, laid out as nl
   bool partitioned = false;      // FP32 lists: fluid-fluid candidates, then the others
   int* vcount = nullptr;         // [n]

@@ -353,14 +353,16 @@ int colloid_drag(Handle* h, double* drag, double* torque) {
 //
 // Bound: the FP64 pipe (64 cycles a warp and instruction), not memory, so
 // what FP64 does not need is off it: the displacement is the difference of FP32
-// offsets against a bound that allows for their rounding (far_bound), the
-// cells' origins come from a table, and FP32 values are rounded on the integer
-// pipe.  512,000 particles: 45 -> 25 us.
+// offsets wherever their rounding cannot change the answer (far_bound; in FP64
+// otherwise, and for particles without a cell, whose offset is the position),
+// the cells' origins come from a table, and FP32 values are rounded on the
+// integer pipe.  512,000 particles: 45 -> 25 us.
 template <int D>
 __global__ void k_kdw_reuse(Consts k, double dt, double4_32a* __restrict__ x,
                             double4_32a* __restrict__ v, const double4_32a* __restrict__ f,
                             const int* __restrict__ sid, double* __restrict__ ct,
-                            const double* __restrict__ act, const float4* __restrict__ off_ref,
+                            const double* __restrict__ act, const double4_32a* __restrict__ x_ref,
+                            const float4* __restrict__ off_ref,
                             const int* __restrict__ cell_of, float4* __restrict__ off,
                             float2* __restrict__ wd, int* __restrict__ flag) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -423,7 +425,17 @@ __global__ void k_kdw_reuse(Consts k, double dt, double4_32a* __restrict__ x,
       dx -= k.le_afff * ref.w;
       if (s >= 0 && (xs[1] < k.min_phys[1] || xs[1] >= k.max_phys[1])) far = true;
     }
-    far = far || dx * dx + dy * dy + dz * dz > k.far2f;
+    const float d2 = dx * dx + dy * dy + dz * dz;
+    const bool meshed = cell < k.ncell;
+    if (meshed && d2 > k.far2f) {
+      far = true;
+    } else if (!far && (!meshed || d2 > k.near2f)) {
+      const double4_32a xr = x_ref[i];
+      double ex = xs[0] - xr.x;
+      const double ey = xs[1] - xr.y, ez = (D == 3) ? xs[2] - xr.z : 0.0;
+      if (k.le) ex -= k.le_aff * (xr.y - k.le_y0);
+      far = ex * ex + ey * ey + ez * ez > k.far2;
+    }
     off[i] = make_float4(of[0], of[1], of[2], __int_as_float(s));
     if (wd != nullptr && k.wall_axis >= 0) {
       const double xa = k.wall_axis == 0 ? xs[0] : (k.wall_axis == 1 ? xs[1] : xs[2]);
@@ -477,10 +489,10 @@ int kick_drift_reuse(Handle* h, double dt) {
   double* ct = h->p.Newtonian ? nullptr : h->ct;
   if (h->k.d == 3)
     k_kdw_reuse<3><<<gb, tb, 0, h->stream>>>(h->k, dt, h->x, h->v, h->f, h->sid, ct, h->act,
-                                             h->off_ref, h->cell_of, h->off, h->wd, h->d_rebuild);
+                                             h->x_ref, h->off_ref, h->cell_of, h->off, h->wd, h->d_rebuild);
   else
     k_kdw_reuse<2><<<gb, tb, 0, h->stream>>>(h->k, dt, h->x, h->v, h->f, h->sid, ct, h->act,
-                                             h->off_ref, h->cell_of, h->off, h->wd, h->d_rebuild);
+                                             h->x_ref, h->off_ref, h->cell_of, h->off, h->wd, h->d_rebuild);
   h->launches++;
   return cuda_check(h, cudaGetLastError(), "kick-drift launch") ? MCFG_ECUDA : MCFG_OK;
 }

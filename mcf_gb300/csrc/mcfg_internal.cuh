@@ -438,14 +438,14 @@ __device__ __forceinline__ double halved(double a) {
 }
 
 // a < b on the integer pipe (an FP64 comparison is an instruction of the narrow
-// pipe).  As the comparison but for NaN (past every number) and the two zeros
-// (-0 before +0); a caller's result must not depend on those.
-__device__ __forceinline__ bool less64(double a, double b) {
-  long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
-  ia ^= (ia >> 63) & 0x7fffffffffffffffll;
-  ib ^= (ib >> 63) & 0x7fffffffffffffffll;
-  return ia < ib;
+// pipe): magnitudes as whole numbers, negated below zero, so that the two zeros
+// are equal.  As the comparison but for NaN (beyond the infinities); a caller's
+// result must not depend on that.
+__device__ __forceinline__ long long order64(double a) {
+  const long long i = __double_as_longlong(a), s = i >> 63;
+  return ((i & 0x7fffffffffffffffll) ^ s) - s;
 }
+__device__ __forceinline__ bool less64(double a, double b) { return order64(a) < order64(b); }
 
 // Philox4x32-10, Salmon et al., SC'11 ("Parallel random numbers: as easy as
 // 1, 2, 3"): multipliers and Weyl key increments of the published algorithm.

@@ -13,8 +13,7 @@ namespace mcfg {
 
 // Periodic wrap of one coordinate, particles_adjust_particles.F90:150-161,
 // 268-279: x < min -> x + length; then x >= max -> x - length.  Solid-wall
-// faces only clamp wall particles to the total domain.  (-0 wraps to L and back
-// to 0, NaN stays NaN.)
+// faces only clamp wall particles to the total domain.  (NaN stays NaN.)
 __device__ __forceinline__ void wrap_axis(const Consts& k, int a,
                                           int sid, double& x, double& v) {
   if (less64(x, k.min_phys[a])) {

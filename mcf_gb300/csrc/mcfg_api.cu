@@ -61,7 +61,7 @@ static int status_copy_async(Handle* h) {
                  "status buffer"))
     return MCFG_ECUDA;
   Handle::HostStatus* hs = h->h_status;
-  if (cuda_check(h, cudaMemcpyAsync(&hs->err, h->d_err, sizeof hs->err, cudaMemcpyDeviceToHost,
+  if (cuda_check(h, cudaMemcpyAsync(hs->err, h->d_err, sizeof hs->err, cudaMemcpyDeviceToHost,
                                     h->stream),
                  "error flag copy") ||
       cuda_check(h, cudaMemcpyAsync(hs->stats, h->d_stats, sizeof hs->stats,
@@ -76,21 +76,26 @@ static int status_copy_async(Handle* h) {
 
 // the status words copied by status_copy_async, after the stream's sync
 static int status_evaluate(Handle* h) {
-  const unsigned e = h->h_status->err;
+  const unsigned e = h->h_status->err[0];
   int st[4];
   for (int q = 0; q < 4; ++q) st[q] = h->h_status->stats[q];
   const unsigned long long pairs = h->h_status->pairs;
   resolve_phases(h);
   h->max_neigh = st[1];
+  if (e & kErrNeighOverflow)  // the lists counted were cut
+    h->max_neigh = std::max(st[1], (int)h->h_status->err[kErrWordNeigh]);
   h->num_pairs = (int64_t)pairs;
   if (e) {
-    cudaMemsetAsync(h->d_err, 0, sizeof(unsigned), h->stream);
-    if (e & kErrNeighOverflow) {
+    cudaMemsetAsync(h->d_err, 0, sizeof(unsigned) * kErrWords, h->stream);
+    if (e & (kErrNeighOverflow | kErrKeptOverflow)) {
+      // a kept list that was cut may leave the step's own list short: it comes first
+      const bool kept = (e & kErrKeptOverflow) != 0;
       char buf[200];
       snprintf(buf, sizeof buf,
-               "neighbour list overflow: a particle has %d candidates, capacity %d "
+               "neighbour list overflow: a particle has %u candidates%s, capacity %d "
                "(raise mcfg_params.reserved[0])",
-               st[1], h->neigh_cap);
+               h->h_status->err[kept ? kErrWordKept : kErrWordNeigh],
+               kept ? " within the cut-off and the skin" : "", kept ? h->vcap : h->neigh_cap);
       return set_error(h, MCFG_EOVERFLOW, buf);
     }
     if (e & kErrCellOverflow)
@@ -569,7 +574,7 @@ int ensure_capacity(Handle* h, int64_t n64) {
         (rc = dalloc(h, &h->cell_start, (size_t)nbins + 2)) ||
         (rc = dalloc(h, &h->scan_part, (size_t)ntiles + 1)) ||
         (rc = dalloc(h, &h->red, (size_t)1024 * 13 + 64)) ||
-        (rc = dalloc(h, &h->d_err, 1)) || (rc = dalloc(h, &h->d_stats, 4)) ||
+        (rc = dalloc(h, &h->d_err, kErrWords)) || (rc = dalloc(h, &h->d_stats, 4)) ||
         (rc = dalloc(h, &h->d_pairs, 1)))
       return rc;
     if (h->k.reuse) {
@@ -622,7 +627,8 @@ int ensure_capacity(Handle* h, int64_t n64) {
     if (cuda_check(h, cudaGetLastError(), "cell origins")) return MCFG_ECUDA;
     h->up_cap = cap;
     h->cap_n = n;
-    if (cuda_check(h, cudaMemsetAsync(h->d_err, 0, sizeof(unsigned), h->stream), "memset err"))
+    if (cuda_check(h, cudaMemsetAsync(h->d_err, 0, sizeof(unsigned) * kErrWords, h->stream),
+                   "memset err"))
       return MCFG_ECUDA;
   }
   return MCFG_OK;

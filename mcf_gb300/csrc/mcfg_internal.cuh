@@ -31,7 +31,11 @@ enum DevErr : unsigned {
   kErrCellOverflow = 2u,    // a cell holds more than kMaxCellCount particles
   kErrZeroDensity = 4u,     // non-positive density met in a pair
   kErrNonFinite = 8u,       // NaN/Inf produced
+  kErrKeptOverflow = 16u,   // capacity of the list kept between steps exceeded
 };
+// the words of Handle::d_err behind the bitmask: the longest list met that did
+// not fit, a step's and the kept one's (they last until the error is reported)
+enum DevErrWord { kErrWordNeigh = 1, kErrWordKept = 2, kErrWords = 3 };
 
 // Constants of one configuration, passed by value to kernels.
 struct Consts {
@@ -142,7 +146,7 @@ struct Handle {
   // device status words (error flags, list statistics, pair count) copied
   // to pinned memory behind a host step, read after its one synchronisation
   struct HostStatus {
-    unsigned err;
+    unsigned err[kErrWords];
     int stats[4];
     unsigned long long pairs;
   };
@@ -231,7 +235,7 @@ struct Handle {
   float2* wd = nullptr;      // FP32 path: signed distances to the wall-axis faces
   // ---- reductions & errors ----
   double* red = nullptr;     // block partials
-  unsigned* d_err = nullptr; // device error bitmask
+  unsigned* d_err = nullptr; // device error bitmask and list lengths [kErrWords]
   int* d_stats = nullptr;    // [0] outside count, [1] max neigh, [2] pairs lo
   unsigned long long* d_pairs = nullptr;
   void* h_pinned = nullptr;  // small pinned staging

@@ -45,7 +45,7 @@ constexpr int kMaskRows = 32;  // candidate chunks a warp notes between two emis
 // and count = fluid-fluid | other << 16.  EXACT: the separation is formed as
 // the density sweep forms it, so that lim decides alike (a step's own FP32
 // list); the other lists have slack in lim and save that addition.
-// gate: return at once when *gate is zero (no rebuild due).
+// gate: the list is the kept one; return at once when *gate is zero (no rebuild due).
 //
 // Bound: instruction issue (a 3D particle meets 27 cells of ~28 particles, of
 // which ~113 are pairs).  So a chunk of 32 candidates is staged once in shared
@@ -60,8 +60,7 @@ template <int D, bool EXACT>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     k_scan(Consts k, const int* __restrict__ gate, const int* __restrict__ cell_start,
            const float4* __restrict__ off, float lim, uint16_t* __restrict__ list,
-           int* __restrict__ count, int cap, int partition, unsigned* __restrict__ err,
-           int* __restrict__ stats) {
+           int* __restrict__ count, int cap, int partition, unsigned* __restrict__ err) {
   if (gate && *gate == 0) return;
   constexpr int CENTER = (D == 3) ? 13 : 4;
   __shared__ NbTable tab[kWarpsPerBlock];
@@ -211,8 +210,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
         if (cnt + cnt_o > cap) {
           // the counts are cut to what fits (every entry below them holds a
           // candidate of this particle), the overflow is reported
-          atomicOr(err, kErrNeighOverflow);
-          atomicMax(&stats[1], cnt + cnt_o);
+          atomicOr(err, gate ? kErrKeptOverflow : kErrNeighOverflow);
+          atomicMax(&err[gate ? kErrWordKept : kErrWordNeigh], (unsigned)(cnt + cnt_o));
           cnt = min(cnt, cap);
           cnt_o = min(cnt_o, cap - cnt);
         }
@@ -333,7 +332,10 @@ __global__ void __launch_bounds__(kReuseTPB)
     }
   }
   if (fin) {
-    if (kept > cap) atomicOr(err, kErrNeighOverflow);
+    if (kept > cap) {
+      atomicOr(err, kErrNeighOverflow);
+      atomicMax(&err[kErrWordNeigh], (unsigned)kept);
+    }
     my_max = kept;
     kept = min(kept, cap);
     ncount[fi] = kept;
@@ -1211,7 +1213,7 @@ static int scan_launch(Handle* h, const int* gate, float lim, uint16_t* list, in
 #define LAUNCH_S(DD, EX)                                                                          \
   k_scan<DD, EX><<<g, kWarpsPerBlock * 32, 0, h->stream>>>(h->k, gate, h->cell_start, h->off, lim, \
                                                            list, count, cap, partition ? 1 : 0,    \
-                                                           h->d_err, h->d_stats)
+                                                           h->d_err)
   if (h->k.d == 3) {
     if (exact) LAUNCH_S(3, true); else LAUNCH_S(3, false);
   } else {

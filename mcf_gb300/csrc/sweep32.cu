@@ -264,6 +264,7 @@ __global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 5)
     const int kept = kff + ko + idle;
     if (kept > cap) {
       atomicOr(err, kErrNeighOverflow);
+      atomicMax(&err[kErrWordNeigh], (unsigned)kept);
       kff = min(kff, cap);
       ko = min(ko, cap - kff);
     }

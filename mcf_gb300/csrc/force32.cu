@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kReuseTPB, 4)
   // lanes past the last particle stay for the block's end, with an empty list
   const int i = S == 1 ? gt : min(gt / S, n - 1);
   const int nc = S == 1 || gt / S < n ? ncount[i] : 0;
-  const int nff = nc & 0xffff, no = nc >> 16;
+  const int nff = first_count(nc), no = second_count(nc);
   // the lane's octets: n0 of the first segment, then those of the second
   const int n0 = max(0, (nff + 7) / 8 - lane_s + S - 1) / S;
   const int nk = n0 + max(0, (no + 7) / 8 - lane_s + S - 1) / S;

@@ -25,6 +25,12 @@ __device__ __forceinline__ size_t down_at(int r, int cap, int n, int i) {
   return ((unsigned long long)(unsigned)(list_octets(cap) - 1 - (r >> 3)) * (unsigned)n + i) * 8 +
          (r & 7);
 }
+// the packed lengths of a list's two segments (up to 27 x 2048 entries each)
+__device__ __forceinline__ int pack_counts(int first, int second) {
+  return (int)((unsigned)first | ((unsigned)second << 16));
+}
+__device__ __forceinline__ int first_count(int packed) { return packed & 0xffff; }
+__device__ __forceinline__ int second_count(int packed) { return (int)((unsigned)packed >> 16); }
 // logical entry e of a list whose first segment holds nff
 __device__ __forceinline__ size_t entry_at(int e, int nff, int cap, int n, int i) {
   return e < nff ? up_at(e, n, i) : down_at(e - nff, cap, n, i);

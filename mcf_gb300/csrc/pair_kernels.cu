@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
           cnt = min(cnt, cap);
           cnt_o = min(cnt_o, cap - cnt);
         }
-        count[i] = partition ? (cnt | (cnt_o << 16)) : cnt;
+        count[i] = partition ? pack_counts(cnt, cnt_o) : cnt;
       }
     }
   }
@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(kReuseTPB, (NNW && D == 3) ? 4 : 5)
   for (int a = 0; a < 9; ++a) sacc[a] = 0.f;
   // the list's two segments: fluid-fluid pairs, then the others
   const int nc = S == 1 || gt / S < n ? ncount[i] : 0;
-  const int nff = nc & 0xffff, cnt = nff + (nc >> 16);
+  const int nff = first_count(nc), cnt = nff + second_count(nc);
   JData nxt;
   int ent_n1 = 0;
   if (lane_s < cnt)

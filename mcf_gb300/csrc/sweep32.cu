@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 5)
     acc_i = dyn_rho(k, si);  // else the density is constant and the sum unused
     const bool mass = k.rhs_density_type == 1;
     const int vc = vcount[i];
-    const int nff = vc & 0xffff, ntot = nff + (vc >> 16);
+    const int nff = first_count(vc), ntot = nff + second_count(vc);
     const int voct = list_octets(vcap), noct = list_octets(cap);
     const bool in_place = nl == vl;
     const uint4* list4 = reinterpret_cast<const uint4*>(vl);
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 5)
       kff = min(kff, cap);
       ko = min(ko, cap - kff);
     }
-    ncount[fi] = kff | (ko << 16);
+    ncount[fi] = pack_counts(kff, ko);
     my_max = kept;
     my_pairs = (unsigned long long)kept;
     const double mi = m[fi];

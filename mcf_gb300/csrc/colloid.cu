@@ -220,6 +220,7 @@ __global__ void __launch_bounds__(kRigidTPB) k_colloid_rigid(Consts k, RigidArgs
         xf[q] = narrow(xc[q]);
         lf[q] = k.periodic[q] ? narrow(k.len[q]) : INFINITY;
         extent = fmaxf(extent, fmaxf(fabsf(narrow(k.min_phys[q])), fabsf(narrow(k.max_phys[q]))));
+        extent = fmaxf(extent, fabsf(xf[q]));  // (past an open face: anywhere)
       }
       const float reach0 = narrow(rad_c) + 5.0f * narrow(a.hn) + 1e-5f * extent;
       for (int j0 = 0; j0 < nc; j0 += kNearChunk) {

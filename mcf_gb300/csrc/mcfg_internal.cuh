@@ -434,10 +434,10 @@ enum { kForceOnly = 0, kForceBody = 1, kForceBodyKick = 2 };
 // Device helpers
 // ------------------------------------------------------------------------
 
-// half of a positive number, exactly (a multiplication by 0.5 is an FP64
-// instruction; (0.5 f) dt and f (dt / 2) round alike)
+// half of a number, exactly, without an FP64 instruction for positive normal
+// ones ((0.5 f) dt and f (dt / 2) round alike)
 __device__ __forceinline__ double halved(double a) {
-  if (__double2hiint(a) < 0x00200000) return 0.5 * a;
+  if ((unsigned)(__double2hiint(a) - 0x00200000) >= 0x7fd00000u) return 0.5 * a;
   return __hiloint2double(__double2hiint(a) - 0x00100000, __double2loint(a));
 }
 

@@ -270,10 +270,14 @@ __global__ void __launch_bounds__(kReuseTPB, 4)
     const int pid_a = __float_as_int(pa.v.w), pid_b = __float_as_int(pb.v.w);
     const bool both = f_both;
     more = fetch_next();
-    // never taken (offsets hold no such NaN): the branch ends the basic block,
-    // so that the gathers are issued here and not, as the compiler otherwise
-    // orders them, behind this pair's arithmetic (258 instead of 233 us)
-    if (__float_as_int(oi.x) == 0x7fabcdef) break;
+    // never taken (offsets hold no such NaN; one that did would end the run as
+    // a non-finite acceleration does): the branch ends the basic block, so
+    // that the gathers are issued here and not, as the compiler otherwise
+    // orders them, behind this pair's arithmetic (258 instead of 234 us)
+    if (__float_as_int(oi.x) == 0x7fabcdef) {
+      atomicOr(err, kErrNonFinite);
+      break;
+    }
     // a lone last pair: its twin is put out of the support, where every term
     // is an exact zero
     if (!both) hb.r[0] = k.beyondf;

@@ -44,8 +44,9 @@ __device__ __forceinline__ F2 gradw2(const Consts& k, F2 d) {
     g = fma2(splat2(15.0f), mul2(a1, a1), g);
     return mul2(splat2(5.0f * k.coef_gradf), g);
   }
+  // (s om first: zero outside the support, however large s is)
   const F2 om = base2(1.0f, s);
-  return mul2(mul2(splat2(12.0f * k.coef_gradf), s), mul2(om, om));
+  return mul2(splat2(12.0f * k.coef_gradf), mul2(mul2(s, om), om));
 }
 
 // sqrt of a non-negative pair
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(kReuseTPB, 4)
     }
     // a lone last pair: its twin is put out of the support, where every term
     // is an exact zero
-    if (!both) hb.r[0] = k.beyondf;
+    if (!both) hb.r[0] = kBeyond;
     F2 r[3], vij[3];
 #pragma unroll
     for (int a = 0; a < D; ++a) {

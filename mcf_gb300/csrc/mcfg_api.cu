@@ -299,7 +299,6 @@ void make_consts(const mcfg_params& p, Consts& k) {
   }
   k.rc2 = p.cut_off * p.cut_off;
   k.rc2f = (float)k.rc2;
-  k.beyondf = (float)(2.0 * p.cut_off);
   // Lees-Edwards y faces: 3 (2D: 1) more stencil slots for the fourth x
   // cell of the row across the face; the offsets follow the time
   // (boundary_update)

@@ -52,8 +52,6 @@ struct Consts {
   float csf[3];
   double rc2;               // cut_off**2
   float rc2f, rc2f_hi;      // FP32 cut-off^2 and its prefilter bound
-  float beyondf;            // a separation outside the support (2 cut_off): the packed
-                            // sweeps put their padding there
   // neighbour-list reuse (mcfg_params.reserved[1] != 0): the candidates
   // within rc + skin are listed at a rebuild and re-tested every step; a
   // rebuild happens when a particle has moved more than skin/2 since the

@@ -103,8 +103,8 @@ __global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 5)
       auto octet = [&](int o) {
         return list4[(unsigned long long)(unsigned)(up ? o : voct - 1 - o) * (unsigned)n + i];
       };
-      // candidates p .. p + 3: their terms are added, the hits that go to the
-      // force sweep returned as bits
+      // candidates p .. p + 3 (p at least is one): their terms are added, the
+      // hits that go to the force sweep returned as bits
       auto four = [&](int p, const unsigned* e) -> unsigned {
         int j[4];
         float4 o[4];
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 5)
         unsigned ent[4], hits = 0;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          ent[u] = p + u < m_ ? e[u] : e[0];
+          ent[u] = u == 0 || p + u < m_ ? e[u] : e[0];
           j[u] = s_start[(ent[u] >> kLocalBits) * (kReuseTPB / S) + tid / S] +
                  (int)(ent[u] & (kMaxCellCount - 1));
           o[u] = off[j[u]];
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kReuseTPB, S == 1 ? 7 : 5)
           ry[u] = (oi.y - o[u].y) - so.y;
           if (D == 3) rz[u] = (oi.z - o[u].z) - so.z;
           // past the segment's end: out of the support
-          if (p + u >= m_) rx[u] = k.beyondf;
+          if (u > 0 && p + u >= m_) rx[u] = kBeyond;
         }
         F2 w[2];
 #pragma unroll

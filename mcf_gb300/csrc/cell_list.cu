@@ -14,10 +14,11 @@ namespace mcfg {
 // has no real cell.  Same operations as ppm_util_rank3d.F90:422-459: the
 // subtraction comes before the multiplication, FLOOR, then the two
 // corrections at the upper boundary.  No contraction is possible here.
-__device__ __forceinline__ int ppm_axis_cell(double xa, double xmin, double xmax,
+// xmax comes as its bound_key.
+__device__ __forceinline__ int ppm_axis_cell(double xa, double xmin, int64_t xmax_key,
                                              double rdx, int nm) {
   int ia = __double2int_rd(__dmul_rn(__dsub_rn(xa, xmin), rdx));
-  const bool inside = less64(xa, xmax);
+  const bool inside = order64(xa) < xmax_key;
   if (!inside && ia < nm) ia = nm;       // outside above: ghost layer
   if (inside && ia >= nm) ia = nm - 1;   // inside: last real cell
   return (ia >= 0 && ia < nm) ? ia : -1;
@@ -36,7 +37,7 @@ __global__ void k_cell_key(Consts k, const double4_32a* __restrict__ x, int* __r
   bool inside = true;
 #pragma unroll
   for (int a = 0; a < D; ++a) {
-    const int ia = ppm_axis_cell(xs[a], k.xmin[a], k.xmax[a], k.rdx[a], k.nm[a]);
+    const int ia = ppm_axis_cell(xs[a], k.xmin[a], k.xmax_key[a], k.rdx[a], k.nm[a]);
     if (ia < 0) inside = false;
     cell += ia * stride;
     stride *= k.nm[a];

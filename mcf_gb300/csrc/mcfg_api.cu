@@ -296,6 +296,9 @@ void make_consts(const mcfg_params& p, Consts& k) {
     k.periodic[a] = (p.bcdef[2 * a] == MCFG_BC_PERIODIC) ? 1 : 0;
     k.min_phys[a] = p.min_phys[a];
     k.max_phys[a] = p.max_phys[a];
+    k.min_key[a] = bound_key(k.min_phys[a]);
+    k.max_key[a] = bound_key(k.max_phys[a]);
+    k.xmax_key[a] = bound_key(k.xmax[a]);
   }
   k.rc2 = p.cut_off * p.cut_off;
   k.rc2f = (float)k.rc2;
@@ -465,7 +468,7 @@ __global__ void k_update_state(Consts k, int n, const int* __restrict__ slot_of,
         // less than half a period apart (tested on the integer pipe): the same
         // image; the division is for the others
         const double gap = cur[a] - xs[a];
-        if (!less64(fabs(gap), halved(k.len[a]))) {
+        if (__double_as_longlong(fabs(gap)) >= __double_as_longlong(halved(k.len[a]))) {
           const double sh = rint(gap / k.len[a]);
           if (sh != 0.0) xs[a] = xs[a] + sh * k.len[a];
         }
@@ -505,9 +508,9 @@ __global__ void k_download_pos(Consts k, int n, const int* __restrict__ hidx,
   const double4_32a v = x[i];
   double xs[3] = {v.x, v.y, v.z};
   for (int a = 0; a < k.d; ++a) {
-    if (k.bc_lo[a] == MCFG_BC_PERIODIC && less64(xs[a], k.min_phys[a]))
+    if (k.bc_lo[a] == MCFG_BC_PERIODIC && order64(xs[a]) < k.min_key[a])
       xs[a] = __dadd_rn(xs[a], k.len[a]);
-    if (k.bc_hi[a] == MCFG_BC_PERIODIC && !less64(xs[a], k.max_phys[a]))
+    if (k.bc_hi[a] == MCFG_BC_PERIODIC && order64(xs[a]) >= k.max_key[a])
       xs[a] = __dsub_rn(xs[a], k.len[a]);
   }
   double* o = out + (size_t)hidx[i] * k.d;

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <string>
 #include <utility>
@@ -105,6 +106,7 @@ struct Consts {
   int wall_rho_type, wall_noslip_type;
   double init_density;
   double min_phys[3], max_phys[3];
+  int64_t min_key[3], max_key[3], xmax_key[3];  // bound_key of min_phys, max_phys, xmax
   double wall_v[6][3];
   int stress;
   // colloids (boundary particles sid = 1..ncoll)
@@ -439,15 +441,21 @@ __device__ __forceinline__ double halved(double a) {
   return __hiloint2double(__double2hiint(a) - 0x00100000, __double2loint(a));
 }
 
-// a < b on the integer pipe (an FP64 comparison is an instruction of the narrow
-// pipe): magnitudes as whole numbers, negated below zero, so that the two zeros
-// are equal.  As the comparison but for NaN (beyond the infinities); a caller's
-// result must not depend on that.
-__device__ __forceinline__ long long order64(double a) {
-  const long long i = __double_as_longlong(a), s = i >> 63;
-  return ((i & 0x7fffffffffffffffll) ^ s) - s;
+// x < bound as order64(x) < bound_key(bound): whole numbers that compare as the
+// numbers do, for an FP64 comparison is an instruction of the narrow pipe.  -0
+// comes right before +0; the key of a bound at 0 is that of -0, so that both
+// lie on it.  NaN lies beyond the infinities; a caller's result must not depend
+// on that.
+__host__ __device__ __forceinline__ int64_t order64(double a) {
+#ifdef __CUDA_ARCH__
+  const int64_t i = __double_as_longlong(a);
+#else
+  int64_t i;
+  memcpy(&i, &a, sizeof i);
+#endif
+  return i ^ ((i >> 63) & 0x7fffffffffffffffll);
 }
-__device__ __forceinline__ bool less64(double a, double b) { return order64(a) < order64(b); }
+inline int64_t bound_key(double b) { return order64(b == 0.0 ? -0.0 : b); }
 
 // Philox4x32-10, Salmon et al., SC'11 ("Parallel random numbers: as easy as
 // 1, 2, 3"): multipliers and Weyl key increments of the published algorithm.

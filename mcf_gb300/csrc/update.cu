@@ -16,7 +16,7 @@ namespace mcfg {
 // faces only clamp wall particles to the total domain.  (NaN stays NaN.)
 __device__ __forceinline__ void wrap_axis(const Consts& k, int a,
                                           int sid, double& x, double& v) {
-  if (less64(x, k.min_phys[a])) {
+  if (order64(x) < k.min_key[a]) {
     if (k.bc_lo[a] == MCFG_BC_PERIODIC) {
       x = __dadd_rn(x, k.len[a]);
     } else if (k.bc_lo[a] == MCFG_BC_WALL_SOLID) {
@@ -26,7 +26,7 @@ __device__ __forceinline__ void wrap_axis(const Consts& k, int a,
       }
     }
   }
-  if (!less64(x, k.max_phys[a])) {
+  if (order64(x) >= k.max_key[a]) {
     if (k.bc_hi[a] == MCFG_BC_PERIODIC) {
       x = __dsub_rn(x, k.len[a]);
     } else if (k.bc_hi[a] == MCFG_BC_WALL_SOLID) {

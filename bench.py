@@ -412,8 +412,8 @@ def roofline_for(sd, torch, w, prec_idx, peaks, step0, clock_mhz=None):
                          "peak_source": f"nominal: {sms} SMs x 2 DFMA x 2 FLOP x {clk:.0f} MHz"}
     fp32_flops = None
     if not prec_idx and tf.exists():
-        # FP32 (non-tensor) FLOP rate of the FP32 sweep: ncu's FADD + FMUL +
-        # 2 FFMA per particle of the same sweep on 64^3 x this launch's
+        # FP32 (non-tensor) FLOP rate of the FP32 sweep: FLOPs per particle
+        # counted from its source for 64^3 + walls x this launch's
         # particles / its event time, against 128 FP32 lanes x 2 FLOP per
         # clock per SM; beside it the pair-body model of the algorithmic
         # FLOPs (~80 a pair side for the Hu-Adams force, ~25 for the
@@ -428,7 +428,7 @@ def roofline_for(sd, torch, w, prec_idx, peaks, step0, clock_mhz=None):
             info = sd.info()
             pairs = info["num_pairs"] / max(w.n, 1)
             fp32_flops = {"achieved": ach / 1e12, "peak": pk / 1e12, "unit": "TFLOP/s",
-                          "frac": ach / pk, "flop_per_particle_ncu": fl,
+                          "frac": ach / pk, "flop_per_particle_source": fl,
                           "algorithmic_flop_per_particle":
                               (per_pair * pairs) if per_pair else None,
                           "peak_source": f"nominal: {sms} SMs x 128 FP32 lanes x 2 FLOP x "

@@ -942,8 +942,8 @@ void destroy_graphs(Handle* h) {
 
 // run_vv may replay captured steps: list reuse (the rebuild is decided on the
 // device), a candidate list in place, no profiling, and constants that do
-// not change from step to step (no oscillating walls; Lees-Edwards runs
-// without list reuse anyway)
+// not change from step to step (no oscillating walls, no Lees-Edwards faces:
+// their images move with the time)
 static bool graph_eligible(const Handle* h) {
   if (!h->k.reuse || !h->reuse_valid || h->profiling || h->graph_off || h->k.le) return false;
   if (h->k.walls)

@@ -67,8 +67,9 @@ struct ListTail {
 };
 
 // The same for four candidates w at a time of which the bits of `hits` are kept.
-// lut (shared, filled by fill_keep_lut) compacts them: per mask two byte
-// selections of the four and two masks of the kept ones.
+// lut compacts them: per mask two byte selections of the four and two masks of
+// the kept ones (keep_entry; in shared memory, all 16 entries filled and the
+// block's barrier passed before the first append).
 struct QuadTail {
   unsigned long long rest = 0;  // the last count % 4 entries, zero above
   int count = 0;

@@ -350,12 +350,12 @@ int colloid_drag(Handle* h, double* drag, double* torque) {
 // Lees-Edwards faces: from the imposed shear, by more than the bound the
 // host derives) or leaves through a Lees-Edwards face.
 //
-// Bound: the FP64 pipe (64 cycles a warp and instruction), not memory, so
+// Bound: the FP64 pipe (64 cycles a warp and instruction) before memory, so
 // what FP64 does not need is off it: the displacement is the difference of FP32
 // offsets wherever their rounding cannot change the answer (far_bound; in FP64
 // otherwise, and for particles without a cell, whose offset is the position),
 // the cells' origins come from a table, and FP32 values are rounded on the
-// integer pipe.  512,000 particles: 45 -> 25 us.
+// integer pipe.  512,000 particles: 45 -> 25 us (60% of the copy rate).
 template <int D>
 __global__ void k_kdw_reuse(Consts k, double dt, double4_32a* __restrict__ x,
                             double4_32a* __restrict__ v, const double4_32a* __restrict__ f,

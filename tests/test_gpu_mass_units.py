@@ -9,9 +9,9 @@ from mcf_gb300.params import PRECISION_FP32_MIXED, make_params
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("mass", [2.0 ** -122, 2.0 ** -100, 1.0])
+@pytest.mark.parametrize("mass", [2.0 ** -122, 1.0])
 @pytest.mark.parametrize("kernel", [1, 2])
-@pytest.mark.parametrize("n", [9, 6000, 25000])
+@pytest.mark.parametrize("n", [9, 25000, 80000])
 def test_mass_density(gpu_lib, n, kernel, mass):
     # particles per unit volume as in a lattice of spacing `unit`
     from oracle.oracle import Oracle

@@ -16,8 +16,8 @@ STEPS = 4  # half a skin is reached at the end of the fourth
 @pytest.mark.parametrize("replayed", [False, True])
 @pytest.mark.parametrize("precision", [PRECISION_FP64, PRECISION_FP32_MIXED])
 @pytest.mark.parametrize("dim", [2, 3])
-@pytest.mark.parametrize("where", [4.3, 11.0, 4000.3, -70000.7])
-@pytest.mark.parametrize("beyond", [-1e-8, -1e-9, 1e-9, 1e-8])
+@pytest.mark.parametrize("where", [4.3, 4000.3, -70000.7])
+@pytest.mark.parametrize("beyond", [-1e-9, 1e-9])
 def test_rebuild_at_half_the_skin(gpu_lib, beyond, where, dim, precision, replayed):
     L = 12.0
     bc = [BC_PERIODIC] * 6

@@ -12,9 +12,9 @@ TINY = np.finfo(np.float64).tiny
 
 @pytest.mark.parametrize("reuse", [0, 1])
 @pytest.mark.parametrize("precision", [PRECISION_FP64, PRECISION_FP32_MIXED])
-@pytest.mark.parametrize("dim", [2, 3])
 @pytest.mark.parametrize("dt", [TINY, 2 * TINY, 2.0 ** 1000, np.inf])
-def test_kick_of_a_lone_particle(gpu_lib, dt, dim, precision, reuse):
+def test_kick_of_a_lone_particle(gpu_lib, dt, precision, reuse):
+    dim = 3
     p = make_params(num_dim=dim, min_phys=[0.0] * 3, max_phys=[12.0] * 3, min_phys_t=[0.0] * 3,
                     max_phys_t=[12.0] * 3, cut_off=3.0, c=10.0, eta=1.0, dt=1e-4,
                     body_force_type=1, body_force=[2.0, 0.0, 0.0], precision=precision)

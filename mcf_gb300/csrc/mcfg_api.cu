@@ -90,6 +90,7 @@ static int status_evaluate(Handle* h) {
     if (e & (kErrNeighOverflow | kErrKeptOverflow)) {
       // a kept list that was cut may leave the step's own list short: it comes first
       const bool kept = (e & kErrKeptOverflow) != 0;
+      if (kept) h->reuse_valid = false;  // no step goes on with a list that was cut
       char buf[200];
       snprintf(buf, sizeof buf,
                "neighbour list overflow: a particle has %u candidates%s, capacity %d "

@@ -57,6 +57,10 @@ def test_kept_list(gpu_lib, dim, precision, steps):
         g.run_vv(0, steps, 1e-9)
     kept, capacity = _reported(e)
     assert kept == 2 * CROWD - 1 and CROWD < capacity < kept
+    # the cut list is not stepped on with: it is made, and reported, again
+    with pytest.raises(MCFGError) as e:
+        g.run_vv(0, steps, 1e-9)
+    assert _reported(e) == [kept, capacity]
     # room for them: no error
     roomy = _handle(dim, precision, 4 * CROWD, True, 3.15)
     roomy.marching_init_force(0)
